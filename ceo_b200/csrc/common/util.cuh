@@ -67,6 +67,18 @@ __device__ __forceinline__ float block_reduce_max(float v, float* red) {
   return red[32];
 }
 
+// ===================================================== q/k normalisation + coefficient
+// One warp per (token, head).  normalize: qn = q/|q|, kn = k/|k| and lambda = 1, so
+// alpha = 1 - exp(-beta); otherwise qn = q, kn = k and alpha = c(beta, |k|^2) with the
+// small-lambda series of the reference (kernels/cuda/efla.cu:93-115).
+__device__ __forceinline__ float efla_coeff(float beta, float lam) {
+  if (lam <= 1e-6f) {
+    const float bl = beta * lam;
+    return beta * (1.f - bl * (0.5f - bl * (1.f / 6.f - bl * (1.f / 24.f))));
+  }
+  return -expm1f(-beta * lam) / lam;
+}
+
 inline int grid_for(long long n, int per_block, int cap) {
   long long g = (n + per_block - 1) / per_block;
   if (g < 1) g = 1;

@@ -1187,18 +1187,6 @@ efla_bwd_final_kernel(const __grid_constant__ CUtensorMap tm_q,
     dalpha[(static_cast<long long>(tok0) + threadIdx.x) * H + h] = dal[threadIdx.x];
 }
 
-// ===================================================== q/k normalisation + coefficient
-// One warp per (token, head).  normalize: qn = q/|q|, kn = k/|k| and lambda = 1, so
-// alpha = 1 - exp(-beta); otherwise qn = q, kn = k and alpha = c(beta, |k|^2) with the
-// small-lambda series of the reference (kernels/cuda/efla.cu:93-115).
-__device__ __forceinline__ float efla_coeff(float beta, float lam) {
-  if (lam <= 1e-6f) {
-    const float bl = beta * lam;
-    return beta * (1.f - bl * (0.5f - bl * (1.f / 6.f - bl * (1.f / 24.f))));
-  }
-  return -expm1f(-beta * lam) / lam;
-}
-
 // D / 8 lanes share one (token, head) row, eight elements (one 16-byte access) each, so a
 // warp covers 32 / (D / 8) rows at a time.
 template <int LPR>

@@ -21,6 +21,7 @@
 #include "common/check.cuh"
 #include "common/ptx.cuh"
 #include "include/ceo_kernels.h"
+#include "skinny.cuh"
 
 CEO_BOUNDS_TU(gemm)
 
@@ -1221,6 +1222,22 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
     p.epi_mode = epi.mode;
     p.aux = epi.aux;
     p.ld_aux = epi.ld_aux;
+  }
+  // Up to 128 rows, K-major, one plain product: the weight-streaming kernel.  A 128 x 256 tile
+  // hands N / 256 SMs a share of B (8 of 148 for a 2048-wide weight); that kernel cuts B into
+  // 128-row tiles and K-slices that fill the chip: the 97 products of a 1.3B decode step (one
+  // row, 2.4 GB of weights) take 0.97 ms one after the other, and 0.96 ms the whole step when
+  // chained (decode.cu); it was 12 ms.
+  if (fz.kind == 0 && !f8.on && !a_mn_major && !b_mn_major && batch == 1 && !accumulate && !bias &&
+      max_ctas <= 0 && M <= 128 && epi.mode != 2) {
+    SkinnyArgs g = {};
+    g.A = A; g.W = B; g.C = C; g.residual = residual; g.act = epi.mode == 1 ? epi.aux : nullptr;
+    g.lda = lda; g.ldw = ldb; g.ldc = ldc; g.ldr = ldr; g.ldact = epi.ld_aux;
+    g.M = M; g.N = N; g.K = K;
+    g.out_f32 = out_f32;
+    g.alpha = alpha;
+    g.status = status;
+    if (skinny_ok(g)) return skinny_gemm(g, stream);
   }
   // bands of 16 row blocks: a wave of 148 tiles is then ~16 x 9 tiles whose A and B panels
   // both stay in L2 (m-fastest over all rows re-reads A once per ~2 n-blocks)

@@ -82,6 +82,20 @@ int ceo_efla_prep_bwd(const void* dqn, const void* dkn, const void* qn, const vo
                       int D, long long dq_stride, long long dk_stride, int normalize,
                       cudaStream_t stream);
 
+/* ---- token-by-token inference ------------------------------------------------
+ * T tokens of each of B sequences (T = 1, or B = 1; B * T <= 128) through every block, states
+ * updated in place; logits (fp32 [B][vocab], may be NULL) of each sequence's last token.
+ * layers: host array of n_layers x 8 device pointers {ln1.weight, w_qkv (n_proj x hidden), w_o,
+ * ln2.weight, w_up (2F x hidden, gate / up rows interleaved), w_down, state (fp32 (B,H,D,D)),
+ * scalar beta (fp32) or NULL (beta logits are columns P*H*D.. of the projection)}.  All weights
+ * bf16, dense, 16-byte aligned.  ws: bf16 workspace of the sum over {hidden, hidden, n_proj,
+ * H*D, F} of round_up(B*T*width, 128) elements.  Launches 2 + 7 * n_layers (+ 1) kernels. */
+int ceo_decode_tokens(const long long* ids, const void* table, long long vocab,
+                      void* const* layers, int n_layers, const void* final_norm, const void* head,
+                      float* logits, void* ws, int B, int T, int hidden, int H, int D, int P,
+                      int n_proj, int F, int normalize, float eps, int* status,
+                      cudaStream_t stream);
+
 /* ---- normalisation ---------------------------------------------------------- */
 int ceo_norm_bwd_blocks(int rows); /* rows of the partial scratch the bwd kernels need */
 int ceo_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* h_out,

@@ -23,6 +23,7 @@ from collections import OrderedDict
 import torch
 import torch.nn as nn
 
+from ..ops import decode as decode_ops
 from ..ops import efla as efla_ops
 from ..ops import nn as K
 from ..ops.fp8 import Fp8Recipe, fp8_linear
@@ -301,6 +302,10 @@ class EflaLM(nn.Module):
         """token: (B,) ids; states: list of (B,H,d,d) fp32 updated in place -> logits (B,V).
         With the PRISM branch enabled the caches live next to the states: they are attached to
         the ``states`` list on first use (``states.prism``) unless passed explicitly."""
+        if token.is_cuda and token.dim() == 1 and prism_caches is None:
+            out = decode_ops.decode_tokens(self, token[:, None], states)
+            if out is not None:
+                return out
         if prism_caches is None and any(b.prism is not None for b in self.blocks):
             prism_caches = getattr(states, "prism", None)
             if prism_caches is None:
@@ -321,6 +326,25 @@ class EflaLM(nn.Module):
             from ..ops.matmul import gemm
             return gemm(hn, w, out_dtype=torch.float32)   # (B, V) logits on the tcgen05 GEMM
         return hn.float() @ w.float().t()
+
+    @torch.no_grad()
+    def prefill_tokens(self, tokens, states):
+        """The tokens of ONE prompt (a sequence of ids) with the recurrence of ``decode_step``
+        (fp32 state, any length): states (1,H,d,d) updated in place -> logits (1,V) after the
+        last token.  On GPU 128 tokens share a pass over the weights."""
+        ids = torch.as_tensor(tokens, dtype=torch.int64).to(self.embed_tokens.device)
+        out, n = None, ids.numel()
+        step = decode_ops.MAX_ROWS
+        i = 0
+        while ids.is_cuda and i < n:
+            last = i + step >= n
+            out = decode_ops.decode_tokens(self, ids[None, i:i + step], states, want_logits=last)
+            if out is None:
+                break
+            i += step
+        for j in range(i, n):  # CPU, or a model the native loop does not cover
+            out = self.decode_step(ids[j:j + 1], states)
+        return out
 
     # ------------------------------------------------------------ checkpoint name mapping
     def count_parameters(self) -> int:

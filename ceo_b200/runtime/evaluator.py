@@ -101,9 +101,7 @@ class Generator:
                      top_p: float = 1.0, eos_id: int | None = None) -> list[int]:
         ids = list(int(t) for t in prompt_ids) or [0]
         states = self.model.new_states(1, self.device)
-        logits = None
-        for t in ids:  # prefill token by token: the state is all the context there is
-            logits = self.model.decode_step(torch.tensor([t], device=self.device), states)
+        logits = self.model.prefill_tokens(ids, states)  # the state is all the context there is
         out = []
         for _ in range(max_new_tokens):
             if temperature <= 0:
