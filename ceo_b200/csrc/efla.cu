@@ -298,8 +298,13 @@ efla_wy_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 // later waits into no-ops, so the kernel still runs to its end.
 constexpr int SER_THREADS = 288;  // 8 compute warps + 1 copy warp
 
+// SB = buffers of the tiles that leave (state snapshot, U').  With one, the next snapshot waits
+// until the copy engine has read the previous chunk's tiles: a TMA round trip on the serial
+// chain of every chunk.  Two take it off the chain.
+// The backward kernel holds one CTA per SM in any case (registers): it always has two.
+constexpr int BWD_SB = 2;
 struct SerialSync {
-  uint64_t full[2], empty[2], full_u, ready_s, ready_u, st_free;
+  uint64_t full[2], empty[2], ready_s[2], ready_u[2], st_free[2];
   volatile uint32_t dead;
   uint32_t pad;
 };
@@ -320,18 +325,19 @@ __device__ __forceinline__ void serial_sync_init(SerialSync* sy) {
   mbar_init(&sy->full[1], 1);
   mbar_init(&sy->empty[0], 8);
   mbar_init(&sy->empty[1], 8);
-  mbar_init(&sy->full_u, 1);
-  mbar_init(&sy->ready_s, 1);
-  mbar_init(&sy->ready_u, 1);
-  mbar_init(&sy->st_free, 1);
+  for (int i = 0; i < 2; ++i) {
+    mbar_init(&sy->ready_s[i], 1);
+    mbar_init(&sy->ready_u[i], 1);
+    mbar_init(&sy->st_free[i], 1);
+  }
   sy->dead = 0;
   fence_mbar_init();
 }
 
 // Token-major tensors (k, w, u, up, ...) are mapped as matrices [B*T][H*D] with the token
 // stride as leading dimension; the state snapshots as [B*H*n*D][D].
-template <int D>
-__global__ void __launch_bounds__(SER_THREADS, 2)
+template <int D, int SB>
+__global__ void __launch_bounds__(SER_THREADS, SB == 1 || D == 64 ? 2 : 1)
 efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_w,
                       const __grid_constant__ CUtensorMap tm_u,
@@ -345,10 +351,10 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
   uint8_t* smem = align1024(smem_raw);
   uint8_t* Wb = smem;                 // [2][TILE]
   uint8_t* Kb = Wb + 2 * TILE;        // [2][TILE]
-  uint8_t* Us = Kb + 2 * TILE;        // [PANEL]
-  uint8_t* Ss = Us + PANEL;           // [D rows x 128 B]
-  uint8_t* Ups = Ss + D * 128;        // [PANEL]
-  SerialSync* sy = reinterpret_cast<SerialSync*>(Ups + PANEL);
+  uint8_t* Ub = Kb + 2 * TILE;        // [2][PANEL]
+  uint8_t* Sb = Ub + 2 * PANEL;       // [SB][D rows x 128 B]
+  uint8_t* Upb = Sb + SB * D * 128;   // [SB][PANEL]
+  SerialSync* sy = reinterpret_cast<SerialSync*>(Upb + SB * PANEL);
 
   // With p_final the grid has twice the column slices: the second half runs the homogeneous
   // recurrence (U = 0) on the identity, i.e. the span's transfer matrix P = prod (I - K^T W),
@@ -364,33 +370,29 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
   if (warp == 8) {
     if (lane != 0) return;
     // ------------------------------------------------------------------ copy thread
-    auto load_wk = [&](int c) {
+    auto load = [&](int c) {
       const int st = c & 1, tok0 = b * T + c * CH;
-      mbar_arrive_expect_tx(&sy->full[st], 2 * TILE);
+      mbar_arrive_expect_tx(&sy->full[st], 2 * TILE + (ident ? 0 : PANEL));
       tma_tok_tile<D>(Wb + st * TILE, &tm_w, &sy->full[st], h * D, tok0);
+      if (!ident) tma_load_2d(Ub + st * PANEL, &tm_u, &sy->full[st], h * D + v0, tok0);
       tma_tok_tile<D>(Kb + st * TILE, &tm_k, &sy->full[st], h * D, tok0);
     };
-    auto load_u = [&](int c) {
-      mbar_arrive_expect_tx(&sy->full_u, PANEL);
-      tma_load_2d(Us, &tm_u, &sy->full_u, h * D + v0, b * T + c * CH);
-    };
-    load_wk(0);
-    if (!ident) load_u(0);
-    if (n > 1) load_wk(1);
+    load(0);
+    if (n > 1) load(1);
     for (int c = 0; c < n; ++c) {
       if (!ident) {
-        ser_wait(sy, &sy->ready_s, c & 1, status);
-        tma_store_2d(&tm_states, Ss, v0, (bh * n + c) * D);
-        ser_wait(sy, &sy->ready_u, c & 1, status);
-        tma_store_2d(&tm_up, Ups, h * D + v0, b * T + c * CH);
+        const int sb = c % SB, ph = (c / SB) & 1;
+        ser_wait(sy, &sy->ready_s[sb], ph, status);
+        tma_store_2d(&tm_states, Sb + sb * D * 128, v0, (bh * n + c) * D);
+        ser_wait(sy, &sy->ready_u[sb], ph, status);
+        tma_store_2d(&tm_up, Upb + sb * PANEL, h * D + v0, b * T + c * CH);
         bulk_commit();
-        if (c + 1 < n) load_u(c + 1);  // the U tile is free once chunk c's U' exists
-        bulk_wait_read<0>();
-        mbar_arrive(&sy->st_free);
+        bulk_wait_read<SB - 1>();  // chunk c - SB + 1 has left its buffers
+        if (c >= SB - 1) mbar_arrive(&sy->st_free[(c - SB + 1) % SB]);
       }
       if (c + 2 < n) {
         ser_wait(sy, &sy->empty[c & 1], (c >> 1) & 1, status);
-        load_wk(c + 2);
+        load(c + 2);
       }
     }
     bulk_wait<0>();
@@ -412,31 +414,32 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
         sacc[mt][nt][e] = ident ? (row == col ? 1.f : 0.f)
                                 : (s0 ? s0[(static_cast<long long>(bh) * D + row) * D + col] : 0.f);
       }
-  const SwzTile St = swz_tile(Ss, D), Ut = swz_tile(Us, CH), Upt = swz_tile(Ups, CH);
   // resets[b][c] != 0: chunk c starts a new document, the state entering it is zero (the flag
   // of the next chunk is fetched a step ahead, off the serial chain)
   unsigned char rz = resets ? resets[b * n] : 0;
 
   for (int c = 0; c < n; ++c) {
-    const SwzTile Wt = swz_tile(Wb + (c & 1) * TILE, CH), Kt = swz_tile(Kb + (c & 1) * TILE, CH);
+    const int sb = c % SB;
+    const SwzTile Wt = swz_tile(Wb + (c & 1) * TILE, CH), Kt = swz_tile(Kb + (c & 1) * TILE, CH),
+                  Ut = swz_tile(Ub + (c & 1) * PANEL, CH), St = swz_tile(Sb + sb * D * 128, D),
+                  Upt = swz_tile(Upb + sb * PANEL, CH);
     if (rz) {
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) zero_acc<NT>(sacc[mt]);
     }
     if (resets && c + 1 < n) rz = resets[b * n + c + 1];
     // snapshot of the state entering chunk c: bf16 MMA operand + saved for O and backward
-    if (!ident && c > 0) ser_wait(sy, &sy->st_free, (c - 1) & 1, status);
+    if (!ident && c >= SB) ser_wait(sy, &sy->st_free[sb], (c / SB - 1) & 1, status);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) frag_store_swz<NT>(St, r * 16 * MT + mt * 16, cw, sacc[mt]);
     if (!ident) fence_proxy_async_smem();
     compute_bar_sync();
-    if (!ident && threadIdx.x == 0) mbar_arrive(&sy->ready_s);
+    if (!ident && threadIdx.x == 0) mbar_arrive(&sy->ready_s[sb]);
     ser_wait(sy, &sy->full[c & 1], (c >> 1) & 1, status);
     {
       float acc[1][NT][4];
       zero_acc<NT>(acc[0]);
       warp_gemm_swz<1, NT, D, false, true>(acc, Wt, 16 * r, St, cw);
-      if (!ident) ser_wait(sy, &sy->full_u, c & 1, status);
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -448,7 +451,7 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
     }
     if (!ident) fence_proxy_async_smem();
     compute_bar_sync();
-    if (!ident && threadIdx.x == 0) mbar_arrive(&sy->ready_u);
+    if (!ident && threadIdx.x == 0) mbar_arrive(&sy->ready_u[sb]);
     warp_gemm_swz<MT, NT, CH, true, true>(sacc, Kt, r * 16 * MT, Upt, cw);
     __syncwarp();
     if (lane == 0) mbar_arrive(&sy->empty[c & 1]);
@@ -829,12 +832,13 @@ efla_state_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                       const float* __restrict__ ds_final, float* __restrict__ ds0,
                       const unsigned char* __restrict__ resets, int T, int H, int* status) {
   constexpr int NT = 4, MT = D / 64, TILE = (D / 64) * PANEL;
+  constexpr int SB = BWD_SB;
   constexpr int STAGE = 3 * TILE + 2 * PANEL;  // K | Q | W | Dl | dO
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint8_t* dSs = smem + 2 * STAGE;   // [D rows x 128 B]
-  uint8_t* dUps = dSs + D * 128;     // [PANEL]
-  SerialSync* sy = reinterpret_cast<SerialSync*>(dUps + PANEL);
+  uint8_t* dSb = smem + 2 * STAGE;       // [SB][D rows x 128 B]
+  uint8_t* dUpb = dSb + SB * D * 128;    // [SB][PANEL]
+  SerialSync* sy = reinterpret_cast<SerialSync*>(dUpb + SB * PANEL);
 
   const int bh = blockIdx.y, b = bh / H, h = bh - b * H, v0 = blockIdx.x * BV;
   const int n = T / CH;
@@ -861,13 +865,14 @@ efla_state_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
     if (n > 1) load(1);
     for (int i = 0; i < n; ++i) {
       const int c = n - 1 - i;
-      ser_wait(sy, &sy->ready_s, i & 1, status);
-      tma_store_2d(&tm_dstates, dSs, v0, (bh * n + c) * D);
-      ser_wait(sy, &sy->ready_u, i & 1, status);
-      tma_store_2d(&tm_dup, dUps, h * D + v0, b * T + c * CH);
+      const int sb = i % SB, ph = (i / SB) & 1;
+      ser_wait(sy, &sy->ready_s[sb], ph, status);
+      tma_store_2d(&tm_dstates, dSb + sb * D * 128, v0, (bh * n + c) * D);
+      ser_wait(sy, &sy->ready_u[sb], ph, status);
+      tma_store_2d(&tm_dup, dUpb + sb * PANEL, h * D + v0, b * T + c * CH);
       bulk_commit();
-      bulk_wait_read<0>();
-      mbar_arrive(&sy->st_free);
+      bulk_wait_read<SB - 1>();
+      if (i >= SB - 1) mbar_arrive(&sy->st_free[(i - SB + 1) % SB]);
       if (i + 2 < n) {
         ser_wait(sy, &sy->empty[i & 1], (i >> 1) & 1, status);
         load(i + 2);
@@ -891,7 +896,6 @@ efla_state_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         dacc[mt][nt][e] =
             ds_final ? ds_final[(static_cast<long long>(bh) * D + row) * D + col] : 0.f;
       }
-  const SwzTile dSt = swz_tile(dSs, D), dUpt = swz_tile(dUps, CH);
   // a chunk that starts a new document passes no gradient to the chunk before it
   unsigned char rz = resets ? resets[b * n + n - 1] : 0;
 
@@ -900,12 +904,14 @@ efla_state_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
     const SwzTile Kt = swz_tile(st, CH), Qt = swz_tile(st + TILE, CH),
                   Wt = swz_tile(st + 2 * TILE, CH), Dlt = swz_tile(st + 3 * TILE, CH),
                   dOt = swz_tile(st + 3 * TILE + PANEL, CH);
-    if (i > 0) ser_wait(sy, &sy->st_free, (i - 1) & 1, status);
+    const int sb = i % SB;
+    const SwzTile dSt = swz_tile(dSb + sb * D * 128, D), dUpt = swz_tile(dUpb + sb * PANEL, CH);
+    if (i >= SB) ser_wait(sy, &sy->st_free[sb], (i / SB - 1) & 1, status);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) frag_store_swz<NT>(dSt, r * 16 * MT + mt * 16, cw, dacc[mt]);
     fence_proxy_async_smem();
     compute_bar_sync();
-    if (threadIdx.x == 0) mbar_arrive(&sy->ready_s);
+    if (threadIdx.x == 0) mbar_arrive(&sy->ready_s[sb]);
     ser_wait(sy, &sy->full[i & 1], (i >> 1) & 1, status);
     {
       float acc[1][NT][4];
@@ -924,7 +930,7 @@ efla_state_bwd_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
     fence_proxy_async_smem();
     compute_bar_sync();
-    if (threadIdx.x == 0) mbar_arrive(&sy->ready_u);
+    if (threadIdx.x == 0) mbar_arrive(&sy->ready_u[sb]);
     warp_gemm_swz<MT, NT, CH, true, true>(dacc, Qt, r * 16 * MT, dOt, cw);
     warp_gemm_swz<MT, NT, CH, true, true>(dacc, Wt, r * 16 * MT, dUpt, cw);
     __syncwarp();
@@ -1346,10 +1352,10 @@ constexpr int BAR_BYTES = 64;  // up to eight mbarriers
 template <int D> constexpr int tile_bytes() { return (D / 64) * PANEL; }
 template <int D> constexpr int stile_bytes() { return (D / 64) * D * 128; }
 template <int D> constexpr int smem_wy() { return 2 * tile_bytes<D>() + PANEL + CH * GLD * 4 + CH * 4 + BAR_BYTES + 1024; }
-template <int D> constexpr int smem_state_fwd() { return 4 * tile_bytes<D>() + 2 * PANEL + D * 128 + static_cast<int>(sizeof(SerialSync)) + 1024; }
+template <int D, int SB> constexpr int smem_state_fwd() { return 4 * tile_bytes<D>() + 2 * PANEL + SB * (PANEL + D * 128) + static_cast<int>(sizeof(SerialSync)) + 1024; }
 template <int D> constexpr int smem_out() { return 3 * tile_bytes<D>() + stile_bytes<D>() + PANEL + BAR_BYTES + 1024; }
 template <int D> constexpr int smem_bwd_local() { return 4 * tile_bytes<D>() + stile_bytes<D>() + BAR_BYTES + 1024; }
-template <int D> constexpr int smem_state_bwd() { return 2 * (3 * tile_bytes<D>() + 2 * PANEL) + D * 128 + PANEL + static_cast<int>(sizeof(SerialSync)) + 1024; }
+template <int D> constexpr int smem_state_bwd() { return 2 * (3 * tile_bytes<D>() + 2 * PANEL) + BWD_SB * (PANEL + D * 128) + static_cast<int>(sizeof(SerialSync)) + 1024; }
 template <int D> constexpr int smem_bwd_final() { return 6 * tile_bytes<D>() + 2 * stile_bytes<D>() + 3 * PANEL + CH * GLD * 4 + 2 * CH * 4 + BAR_BYTES + 1024; }
 
 template <typename Kern>
@@ -1362,7 +1368,10 @@ static cudaError_t efla_configure() {
   if (cfg) return cudaSuccess;
   cudaError_t e;
   if ((e = set_smem(efla_wy_kernel<D>, smem_wy<D>())) != cudaSuccess) return e;
-  if ((e = set_smem(efla_state_fwd_kernel<D>, smem_state_fwd<D>())) != cudaSuccess) return e;
+  if constexpr (D == 128) {
+    if ((e = set_smem(efla_state_fwd_kernel<D, 1>, smem_state_fwd<D, 1>())) != cudaSuccess) return e;
+  }
+  if ((e = set_smem(efla_state_fwd_kernel<D, 2>, smem_state_fwd<D, 2>())) != cudaSuccess) return e;
   if ((e = set_smem(efla_out_kernel<D>, smem_out<D>())) != cudaSuccess) return e;
   if (D == 128 && (e = set_smem(efla_out_tc_kernel, OUT_TC_SMEM)) != cudaSuccess) return e;
   if ((e = set_smem(efla_bwd_local_kernel<D>, smem_bwd_local<D>())) != cudaSuccess) return e;
@@ -1432,10 +1441,22 @@ static int efla_run_stage(int stage, const EflaTensors& t, int B, int T, int H, 
       MAP(tok(&m[2], I_U, HD));
       MAP(tok(&m[3], I_UP, HD));
       MAP(sta(&m[4], I_STATES));
-      efla_state_fwd_kernel<D><<<dim3(t.p[I_PFINAL] ? 2 * (D / BV) : D / BV, B * H), SER_THREADS,
-                                 smem_state_fwd<D>(), st>>>(
-          m[0], m[1], m[2], m[3], m[4], f32(I_S0), f32(I_SFINAL), f32(I_PFINAL),
-          static_cast<const unsigned char*>(t.p[I_RESETS]), T, H, status);
+      {
+        const dim3 g(t.p[I_PFINAL] ? 2 * (D / BV) : D / BV, B * H);
+        // two buffers of the leaving tiles, unless they (128-wide heads: 130 KB) would leave one
+        // CTA per SM while the grid needs two
+        auto kern = efla_state_fwd_kernel<D, 2>;
+        int smem = smem_state_fwd<D, 2>();
+        if constexpr (D == 128) {
+          if (g.x * g.y > 148) {
+            kern = efla_state_fwd_kernel<D, 1>;
+            smem = smem_state_fwd<D, 1>();
+          }
+        }
+        kern<<<g, SER_THREADS, smem, st>>>(
+            m[0], m[1], m[2], m[3], m[4], f32(I_S0), f32(I_SFINAL), f32(I_PFINAL),
+            static_cast<const unsigned char*>(t.p[I_RESETS]), T, H, status);
+      }
       break;
     case 2:
       if (g_out_tcgen05 && D == 128 && (n & 1) == 0) {  // chunk pairs on the tcgen05 path
