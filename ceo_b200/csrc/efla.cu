@@ -268,7 +268,7 @@ efla_wy_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     uint2 xo;
     *reinterpret_cast<bf162*>(&xo.x) = __floats2bfloat162_rn(x0, x1);
     *reinterpret_cast<bf162*>(&xo.y) = __floats2bfloat162_rn(x2, x3);
-    *reinterpret_cast<uint2*>(xg + i * CH + c) = xo;
+    if (xinv) *reinterpret_cast<uint2*>(xg + i * CH + c) = xo;
   }
   __syncthreads();
   const long long orow = (static_cast<long long>(tok0) + 16 * warp) * H + h;  // row of (B*T*H, D)
@@ -345,7 +345,7 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_states,
                       const float* __restrict__ s0, float* __restrict__ s_final,
                       float* __restrict__ p_final, const unsigned char* __restrict__ resets, int T,
-                      int H, int* status) {
+                      int H, int* status, int segs, int map_pass) {
   constexpr int NT = 4, MT = D / 64, NSL = D / BV, TILE = (D / 64) * PANEL;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -359,10 +359,19 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
   // With p_final the grid has twice the column slices: the second half runs the homogeneous
   // recurrence (U = 0) on the identity, i.e. the span's transfer matrix P = prod (I - K^T W),
   // which context parallelism needs next to the zero-state response.
+  // With segs > 1 the chunks of a sequence are cut into that many spans walked side by side (see
+  // efla_state_segmented).  map_pass: only the spans' maps are wanted (span 0 from s0, the others
+  // from zero and, in the second half of the slices, the transfer matrix); no tile leaves.
+  // Otherwise every span has its incoming state in s0 and only the last one's end is s_final.
   const bool ident = blockIdx.x >= NSL;
-  const int bh = blockIdx.y, b = bh / H, h = bh - b * H, v0 = (blockIdx.x % NSL) * BV;
-  const int n = T / CH;
+  const int bh = blockIdx.y / segs, seg = blockIdx.y - bh * segs;
+  const int b = bh / H, h = bh - b * H, v0 = (blockIdx.x % NSL) * BV;
+  const int nall = T / CH;
+  const int cbeg = seg * nall / segs, n = (seg + 1) * nall / segs - cbeg;
+  const bool quiet = ident || map_pass;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the map pass needs neither the last span's map nor the transfer matrix of the first
+  if (map_pass && (seg == segs - 1 || (ident && seg == 0))) return;
 
   if (threadIdx.x == 0) serial_sync_init(sy);
   __syncthreads();
@@ -371,7 +380,7 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
     if (lane != 0) return;
     // ------------------------------------------------------------------ copy thread
     auto load = [&](int c) {
-      const int st = c & 1, tok0 = b * T + c * CH;
+      const int st = c & 1, tok0 = b * T + (cbeg + c) * CH;
       mbar_arrive_expect_tx(&sy->full[st], 2 * TILE + (ident ? 0 : PANEL));
       tma_tok_tile<D>(Wb + st * TILE, &tm_w, &sy->full[st], h * D, tok0);
       if (!ident) tma_load_2d(Ub + st * PANEL, &tm_u, &sy->full[st], h * D + v0, tok0);
@@ -380,12 +389,12 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
     load(0);
     if (n > 1) load(1);
     for (int c = 0; c < n; ++c) {
-      if (!ident) {
+      if (!quiet) {
         const int sb = c % SB, ph = (c / SB) & 1;
         ser_wait(sy, &sy->ready_s[sb], ph, status);
-        tma_store_2d(&tm_states, Sb + sb * D * 128, v0, (bh * n + c) * D);
+        tma_store_2d(&tm_states, Sb + sb * D * 128, v0, (bh * nall + cbeg + c) * D);
         ser_wait(sy, &sy->ready_u[sb], ph, status);
-        tma_store_2d(&tm_up, Upb + sb * PANEL, h * D + v0, b * T + c * CH);
+        tma_store_2d(&tm_up, Upb + sb * PANEL, h * D + v0, b * T + (cbeg + c) * CH);
         bulk_commit();
         bulk_wait_read<SB - 1>();  // chunk c - SB + 1 has left its buffers
         if (c >= SB - 1) mbar_arrive(&sy->st_free[(c - SB + 1) % SB]);
@@ -403,6 +412,10 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
   const int g = lane >> 2, tg = lane & 3;
   const int r = warp & 3, half = warp >> 2, cw = 32 * half;
   float sacc[MT][NT][4];
+  // map pass: s0 enters span 0 alone; otherwise s0 holds one state per span
+  const float* s_in = s0 && (!map_pass || seg == 0)
+                          ? s0 + static_cast<long long>(map_pass ? bh : blockIdx.y) * D * D
+                          : nullptr;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -412,11 +425,11 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
         const int row = r * 16 * MT + mt * 16 + g + (e >> 1) * 8;
         const int col = v0 + cw + nt * 8 + 2 * tg + (e & 1);
         sacc[mt][nt][e] = ident ? (row == col ? 1.f : 0.f)
-                                : (s0 ? s0[(static_cast<long long>(bh) * D + row) * D + col] : 0.f);
+                                : (s_in ? s_in[static_cast<long long>(row) * D + col] : 0.f);
       }
   // resets[b][c] != 0: chunk c starts a new document, the state entering it is zero (the flag
   // of the next chunk is fetched a step ahead, off the serial chain)
-  unsigned char rz = resets ? resets[b * n] : 0;
+  unsigned char rz = resets ? resets[b * nall + cbeg] : 0;
 
   for (int c = 0; c < n; ++c) {
     const int sb = c % SB;
@@ -427,14 +440,14 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) zero_acc<NT>(sacc[mt]);
     }
-    if (resets && c + 1 < n) rz = resets[b * n + c + 1];
+    if (resets && c + 1 < n) rz = resets[b * nall + cbeg + c + 1];
     // snapshot of the state entering chunk c: bf16 MMA operand + saved for O and backward
-    if (!ident && c >= SB) ser_wait(sy, &sy->st_free[sb], (c / SB - 1) & 1, status);
+    if (!quiet && c >= SB) ser_wait(sy, &sy->st_free[sb], (c / SB - 1) & 1, status);
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) frag_store_swz<NT>(St, r * 16 * MT + mt * 16, cw, sacc[mt]);
-    if (!ident) fence_proxy_async_smem();
+    if (!quiet) fence_proxy_async_smem();
     compute_bar_sync();
-    if (!ident && threadIdx.x == 0) mbar_arrive(&sy->ready_s[sb]);
+    if (!quiet && threadIdx.x == 0) mbar_arrive(&sy->ready_s[sb]);
     ser_wait(sy, &sy->full[c & 1], (c >> 1) & 1, status);
     {
       float acc[1][NT][4];
@@ -449,13 +462,16 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
           sts_bf162(Upt.at(row, col), uu.x - acc[0][nt][2 * hf], uu.y - acc[0][nt][2 * hf + 1]);
         }
     }
-    if (!ident) fence_proxy_async_smem();
+    if (!quiet) fence_proxy_async_smem();
     compute_bar_sync();
-    if (!ident && threadIdx.x == 0) mbar_arrive(&sy->ready_u[sb]);
+    if (!quiet && threadIdx.x == 0) mbar_arrive(&sy->ready_u[sb]);
     warp_gemm_swz<MT, NT, CH, true, true>(sacc, Kt, r * 16 * MT, Upt, cw);
     __syncwarp();
     if (lane == 0) mbar_arrive(&sy->empty[c & 1]);
   }
+  if (!map_pass && seg != segs - 1) return;
+  float* out = (ident ? p_final : s_final) +
+               static_cast<long long>(map_pass ? blockIdx.y : bh) * D * D;
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
@@ -464,9 +480,53 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
       for (int e = 0; e < 4; ++e) {
         const int row = r * 16 * MT + mt * 16 + g + (e >> 1) * 8;
         const int col = v0 + cw + nt * 8 + 2 * tg + (e & 1);
-        (ident ? p_final : s_final)[(static_cast<long long>(bh) * D + row) * D + col] =
-            sacc[mt][nt][e];
+        out[static_cast<long long>(row) * D + col] = sacc[mt][nt][e];
       }
+}
+
+// Incoming state of every span from the spans' maps: s[0] = s0, s[1] = R[0] (span 0 ran from
+// s0), s[j + 1] = P[j] s[j] + R[j].  One CTA per (sequence, head, 8 value columns), the state
+// slice in shared memory; thread (row, half) adds half of the 8 columns of one row in fp32.
+template <int D>
+__global__ void __launch_bounds__(2 * D)
+efla_fold_kernel(const float* __restrict__ s0, const float* __restrict__ P,
+                 const float* __restrict__ R, float* __restrict__ s_in, int segs) {
+  __shared__ float4 ss[D][2];
+  const long long bh = blockIdx.y;
+  const int row = threadIdx.x >> 1, half = threadIdx.x & 1, col = blockIdx.x * 8 + half * 4;
+  const long long cell = static_cast<long long>(row) * D + col;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (s0) s = *reinterpret_cast<const float4*>(s0 + bh * D * D + cell);
+  *reinterpret_cast<float4*>(s_in + bh * segs * D * D + cell) = s;
+  for (int j = 0; j + 1 < segs; ++j) {
+    const long long o = (bh * segs + j) * D * D;
+    float4 acc = *reinterpret_cast<const float4*>(R + o + cell);
+    if (j > 0) {
+      // the whole row of P is requested at once, ahead of the barriers
+      const float4* prow = reinterpret_cast<const float4*>(P + o + static_cast<long long>(row) * D);
+      float4 pr[D / 4];
+#pragma unroll
+      for (int k = 0; k < D / 4; ++k)  // (volatile: the compiler would sink them behind the barriers)
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(pr[k].x), "=f"(pr[k].y), "=f"(pr[k].z), "=f"(pr[k].w)
+                     : "l"(prow + k));
+      __syncthreads();  // the previous step's reads are over
+      ss[row][half] = s;
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < D / 4; ++k) {
+        const float4 pv = pr[k];
+        const float4 a = ss[4 * k][half], b = ss[4 * k + 1][half], c = ss[4 * k + 2][half],
+                     d = ss[4 * k + 3][half];
+        acc.x += pv.x * a.x + pv.y * b.x + pv.z * c.x + pv.w * d.x;
+        acc.y += pv.x * a.y + pv.y * b.y + pv.z * c.y + pv.w * d.y;
+        acc.z += pv.x * a.z + pv.y * b.z + pv.z * c.z + pv.w * d.z;
+        acc.w += pv.x * a.w + pv.y * b.w + pv.z * c.w + pv.w * d.w;
+      }
+    }
+    s = acc;
+    *reinterpret_cast<float4*>(s_in + o + static_cast<long long>(D) * D + cell) = s;
+  }
 }
 
 // ================================================================ forward: O
@@ -1390,9 +1450,64 @@ static int g_out_tcgen05 = 0;
 struct EflaTensors {
   const void* p[25];
   long long stride[6];  // q, k, v, dq, dk, dv
+  int segs = 1;         // spans of the forward state recurrence
+  bool keep_xinv = true;    // false: inference, nobody reads the inverses
+  float* seg_ws = nullptr;  // fp32 [3][B * H * segs][D][D] when segs > 1
 };
 enum { I_Q = 0, I_K, I_V, I_ALPHA, I_W, I_U, I_UP, I_STATES, I_O, I_S0, I_SFINAL, I_DO, I_DLOC,
        I_DUP, I_DSTATES, I_DSFINAL, I_DS0, I_DQ, I_DK, I_DV, I_DALPHA, I_PFINAL, I_STATUS, I_XINV, I_RESETS };
+
+template <int D>
+static void efla_state_launch(const CUtensorMap* m, dim3 g, const float* s0, float* s_final,
+                              float* p_final, const EflaTensors& t, int T, int H, int segs,
+                              int map_pass, cudaStream_t st) {
+  // two buffers of the leaving tiles, unless they (128-wide heads: 130 KB) would leave one
+  // CTA per SM while the grid needs two
+  auto kern = efla_state_fwd_kernel<D, 2>;
+  int smem = smem_state_fwd<D, 2>();
+  if constexpr (D == 128) {
+    if (g.x * g.y > 148) {
+      kern = efla_state_fwd_kernel<D, 1>;
+      smem = smem_state_fwd<D, 1>();
+    }
+  }
+  kern<<<g, SER_THREADS, smem, st>>>(
+      m[0], m[1], m[2], m[3], m[4], s0, s_final, p_final,
+      static_cast<const unsigned char*>(t.p[I_RESETS]), T, H,
+      static_cast<int*>(const_cast<void*>(t.p[I_STATUS])), segs, map_pass);
+}
+
+// The forward recurrence with few chains and many chunks.  A chunk's step is a chain of two
+// products and two barriers (about 1.25 us) whatever the chip has left over, so with 16 chains
+// and 1024 chunks the plain kernel leaves 130 SMs idle for most of the layer.  Over a span of
+// chunks the recurrence is affine, S_out = P S_in + R: all spans' (P, R) side by side, a short
+// fp32 fold over the spans, then the real pass over all spans side by side.  Three times the
+// arithmetic, 2 / segs of the serial steps: 16 chains of 64, 65536 tokens, 1.27 ms -> 0.42 ms a
+// layer (10 spans); 16 chains of 128, 4096 tokens, 123 us -> 78 us (5 spans).
+template <int D>
+static int efla_state_segmented(const CUtensorMap* m, const EflaTensors& t, int B, int T, int H,
+                                cudaStream_t st) {
+  const int G = t.segs;
+  const long long one = static_cast<long long>(B) * H * G * D * D;
+  float *R = t.seg_ws, *P = R + one, *s_in = P + one;
+  const float* s0 = static_cast<const float*>(t.p[I_S0]);
+  efla_state_launch<D>(m, dim3(2 * (D / BV), B * H * G), s0, R, P, t, T, H, G, 1, st);
+  efla_fold_kernel<D><<<dim3(D / 8, B * H), 2 * D, 0, st>>>(s0, P, R, s_in, G);
+  efla_state_launch<D>(m, dim3(D / BV, B * H * G), s_in,
+                       static_cast<float*>(const_cast<void*>(t.p[I_SFINAL])), nullptr, t, T, H, G,
+                       0, st);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Spans for a forward call: as many as keep the map pass (2 (D / 64) CTAs per span and chain)
+// within the two CTAs per SM that are resident, at least 6 chunks each; 1 (the plain kernel)
+// below three, where the extra passes eat the gain.
+static int efla_segments(int B, int T, int H, int D) {
+  const int n = T / CH, per_span = 2 * (D / BV) * B * H;
+  int g = 1 + 296 / per_span;
+  if (g > n / 6) g = n / 6;
+  return g >= 3 ? g : 1;
+}
 
 template <int D>
 static int efla_run_stage(int stage, const EflaTensors& t, int B, int T, int H, cudaStream_t st) {
@@ -1431,7 +1546,7 @@ static int efla_run_stage(int stage, const EflaTensors& t, int B, int T, int H, 
     case 0:
       MAP(tokp(&m[0], I_K, t.stride[1]));
       MAP(tokp(&m[1], I_V, t.stride[2]));
-      if (!t.p[I_XINV]) return -5;
+      if (!t.p[I_XINV] && t.keep_xinv) return -5;
       efla_wy_kernel<D><<<gpar, 128, smem_wy<D>(), st>>>(m[0], m[1], f32(I_ALPHA), b16(I_W),
                                                          b16(I_U), b16(I_XINV), T, H, status);
       break;
@@ -1441,22 +1556,10 @@ static int efla_run_stage(int stage, const EflaTensors& t, int B, int T, int H, 
       MAP(tok(&m[2], I_U, HD));
       MAP(tok(&m[3], I_UP, HD));
       MAP(sta(&m[4], I_STATES));
-      {
-        const dim3 g(t.p[I_PFINAL] ? 2 * (D / BV) : D / BV, B * H);
-        // two buffers of the leaving tiles, unless they (128-wide heads: 130 KB) would leave one
-        // CTA per SM while the grid needs two
-        auto kern = efla_state_fwd_kernel<D, 2>;
-        int smem = smem_state_fwd<D, 2>();
-        if constexpr (D == 128) {
-          if (g.x * g.y > 148) {
-            kern = efla_state_fwd_kernel<D, 1>;
-            smem = smem_state_fwd<D, 1>();
-          }
-        }
-        kern<<<g, SER_THREADS, smem, st>>>(
-            m[0], m[1], m[2], m[3], m[4], f32(I_S0), f32(I_SFINAL), f32(I_PFINAL),
-            static_cast<const unsigned char*>(t.p[I_RESETS]), T, H, status);
-      }
+      if (t.segs > 1)
+        return efla_state_segmented<D>(m, t, B, T, H, st);
+      efla_state_launch<D>(m, dim3(t.p[I_PFINAL] ? 2 * (D / BV) : D / BV, B * H), f32(I_S0),
+                           f32(I_SFINAL), f32(I_PFINAL), t, T, H, 1, 0, st);
       break;
     case 2:
       if (g_out_tcgen05 && D == 128 && (n & 1) == 0) {  // chunk pairs on the tcgen05 path
@@ -1536,13 +1639,27 @@ extern "C" int ceo_efla_set_tcgen05(int on) {
   return 0;
 }
 
-extern "C" int ceo_efla_fwd(const void* q, const void* k, const void* v, const float* alpha,
-                            const float* s0, void* w, void* up, void* states, void* xinv, void* o,
-                            float* s_final, const unsigned char* resets, int B, int T, int H,
-                            int D, long long q_stride, long long k_stride, long long v_stride,
-                            int* status, cudaStream_t stream) {
+// Spans the forward recurrence is cut into for this shape (1: no workspace needed); 0 for a
+// shape that is refused.
+extern "C" int ceo_efla_fwd_segments(int B, int T, int H, int D) {
+  if (!efla_args_ok(B, T, H, D, 0, 0, 0)) return 0;
+  return efla_segments(B, T, H, D);
+}
+
+static int efla_fwd_run(const void* q, const void* k, const void* v, const float* alpha,
+                        const float* s0, void* w, void* up, void* states, void* xinv, void* o,
+                        float* s_final, const unsigned char* resets, int B, int T, int H, int D,
+                        long long q_stride, long long k_stride, long long v_stride, int segs,
+                        float* seg_ws, int* status, cudaStream_t stream, bool keep_xinv = true) {
   if (!efla_args_ok(B, T, H, D, q_stride, k_stride, v_stride)) return -5;
+  if (segs < 1 || segs > T / CH || static_cast<long long>(B) * H * segs > 65535 ||
+      (segs > 1 && (!seg_ws || ((reinterpret_cast<uintptr_t>(seg_ws) |
+                                 reinterpret_cast<uintptr_t>(s0)) & 15))))
+    return -5;
   EflaTensors t = {};
+  t.segs = segs;
+  t.seg_ws = seg_ws;
+  t.keep_xinv = keep_xinv;
   t.p[I_Q] = q; t.p[I_K] = k; t.p[I_V] = v; t.p[I_ALPHA] = alpha; t.p[I_W] = w;
   t.p[I_U] = o;  // U is staged in `o` (same shape, overwritten by the last kernel)
   t.p[I_UP] = up; t.p[I_STATES] = states; t.p[I_O] = o; t.p[I_S0] = s0; t.p[I_SFINAL] = s_final;
@@ -1554,6 +1671,25 @@ extern "C" int ceo_efla_fwd(const void* q, const void* k, const void* v, const f
     if (rc) return rc;
   }
   return 0;
+}
+
+extern "C" int ceo_efla_fwd_seg(const void* q, const void* k, const void* v, const float* alpha,
+                                const float* s0, void* w, void* up, void* states, void* xinv,
+                                void* o, float* s_final, const unsigned char* resets, int segs,
+                                float* seg_ws, int B, int T, int H, int D, long long q_stride,
+                                long long k_stride, long long v_stride, int* status,
+                                cudaStream_t stream) {
+  return efla_fwd_run(q, k, v, alpha, s0, w, up, states, xinv, o, s_final, resets, B, T, H, D,
+                      q_stride, k_stride, v_stride, segs, seg_ws, status, stream, xinv != nullptr);
+}
+
+extern "C" int ceo_efla_fwd(const void* q, const void* k, const void* v, const float* alpha,
+                            const float* s0, void* w, void* up, void* states, void* xinv, void* o,
+                            float* s_final, const unsigned char* resets, int B, int T, int H,
+                            int D, long long q_stride, long long k_stride, long long v_stride,
+                            int* status, cudaStream_t stream) {
+  return efla_fwd_run(q, k, v, alpha, s0, w, up, states, xinv, o, s_final, resets, B, T, H, D,
+                      q_stride, k_stride, v_stride, 1, nullptr, status, stream);
 }
 
 extern "C" int ceo_efla_bwd(const void* q, const void* k, const void* v, const float* alpha,

@@ -53,6 +53,15 @@ int ceo_efla_fwd(const void* q, const void* k, const void* v, const float* alpha
                  void* w, void* up, void* states, void* xinv, void* o, float* s_final,
                  const unsigned char* resets, int B, int T, int H, int D, long long q_stride,
                  long long k_stride, long long v_stride, int* status, cudaStream_t stream);
+/* The same with the state recurrence cut into `segs` spans that run side by side (few chains and
+ * many chunks); seg_ws: fp32 [3][B*H*segs][D][D], 16-byte aligned (so must s0 be).  segs = 1 is
+ * ceo_efla_fwd, except that xinv may be NULL (no backward pass); ceo_efla_fwd_segments() is the count that suits a shape. */
+int ceo_efla_fwd_segments(int B, int T, int H, int D);
+int ceo_efla_fwd_seg(const void* q, const void* k, const void* v, const float* alpha,
+                     const float* s0, void* w, void* up, void* states, void* xinv, void* o,
+                     float* s_final, const unsigned char* resets, int segs, float* seg_ws, int B,
+                     int T, int H, int D, long long q_stride, long long k_stride,
+                     long long v_stride, int* status, cudaStream_t stream);
 int ceo_efla_bwd(const void* q, const void* k, const void* v, const float* alpha, const void* w,
                  const void* up, const void* states, const void* xinv, const void* dO,
                  const float* ds_final, void* dloc, void* dup, void* dstates, void* dq, void* dk,

@@ -37,6 +37,26 @@ def _tok_stride(t: torch.Tensor) -> int:
     return t.stride(1)
 
 
+def _fwd(q_ptr, k_ptr, v_ptr, alpha, s0, w, up, states, xinv, o, s_final, resets, B, T, H, d,
+         q_stride, k_stride, v_stride):
+    """The forward kernels; the state recurrence in spans where the shape has few chains."""
+    L = _lib.lib()
+    st = _lib.status_word(o.device).data_ptr()
+    segs = L.ceo_efla_fwd_segments(B, T, H, d)
+    if segs > 1 and (s0 is None or s0.data_ptr() % 16 == 0):
+        ws = torch.empty(3 * B * H * segs * d * d, dtype=torch.float32, device=o.device)
+        _lib.check(L.ceo_efla_fwd_seg(q_ptr, k_ptr, v_ptr, alpha.data_ptr(), _lib.ptr(s0),
+                                      w.data_ptr(), up.data_ptr(), states.data_ptr(),
+                                      xinv.data_ptr(), o.data_ptr(), s_final.data_ptr(),
+                                      _lib.ptr(resets), segs, ws.data_ptr(), B, T, H, d, q_stride,
+                                      k_stride, v_stride, st, _lib.stream()), "ceo_efla_fwd_seg")
+        return
+    _lib.check(L.ceo_efla_fwd(q_ptr, k_ptr, v_ptr, alpha.data_ptr(), _lib.ptr(s0), w.data_ptr(),
+                              up.data_ptr(), states.data_ptr(), xinv.data_ptr(), o.data_ptr(),
+                              s_final.data_ptr(), _lib.ptr(resets), B, T, H, d, q_stride, k_stride,
+                              v_stride, st, _lib.stream()), "ceo_efla_fwd")
+
+
 class _DeltaRuleFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, alpha, s0, resets=None):
@@ -53,15 +73,8 @@ class _DeltaRuleFn(torch.autograd.Function):
         states = torch.empty(B, H, n, d, d, dtype=torch.bfloat16, device=dev)
         xinv = torch.empty(B, H, n, CHUNK, CHUNK, dtype=torch.bfloat16, device=dev)
         s_final = torch.empty(B, H, d, d, dtype=torch.float32, device=dev)
-        L = _lib.lib()
-        st = _lib.status_word(dev).data_ptr()
-        _lib.check(L.ceo_efla_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), alpha.data_ptr(),
-                                  _lib.ptr(s0), w.data_ptr(), up.data_ptr(), states.data_ptr(),
-                                  xinv.data_ptr(),
-                                  o.data_ptr(), s_final.data_ptr(), _lib.ptr(resets), B, T, H, d,
-                                  _tok_stride(q), _tok_stride(k), _tok_stride(v), st,
-                                  _lib.stream()),
-                   "ceo_efla_fwd")
+        _fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), alpha, s0, w, up, states, xinv, o, s_final,
+             resets, B, T, H, d, _tok_stride(q), _tok_stride(k), _tok_stride(v))
         ctx.save_for_backward(q, k, v, alpha, w, up, states, xinv)
         ctx.has_s0 = s0 is not None
         return o, s_final
@@ -134,13 +147,8 @@ class _EflaQKVFn(torch.autograd.Function):
         states = torch.empty(B, H, n, d, d, dtype=torch.bfloat16, device=dev)
         xinv = torch.empty(B, H, n, CHUNK, CHUNK, dtype=torch.bfloat16, device=dev)
         s_final = torch.empty(B, H, d, d, dtype=torch.float32, device=dev)
-        st = _lib.status_word(dev).data_ptr()
-        _lib.check(L.ceo_efla_fwd(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), alpha.data_ptr(),
-                                  _lib.ptr(s0), w.data_ptr(), up.data_ptr(), states.data_ptr(),
-                                  xinv.data_ptr(),
-                                  o.data_ptr(), s_final.data_ptr(), _lib.ptr(resets), B, T, H, d,
-                                  H * d, H * d, ts,
-                                  st, _lib.stream()), "ceo_efla_fwd")
+        _fwd(qn.data_ptr(), kn.data_ptr(), v.data_ptr(), alpha, s0, w, up, states, xinv, o,
+             s_final, resets, B, T, H, d, H * d, H * d, ts)
         ctx.save_for_backward(qkv, beta, qn, kn, rq, rk, alpha, w, up, states, xinv)
         ctx.cfg = (normalize, scalar, s0 is not None)
         return o, s_final
@@ -296,13 +304,8 @@ class _EflaProjFn(torch.autograd.Function):
         states = torch.empty(B, H, n, d, d, dtype=torch.bfloat16, device=dev)
         xinv = torch.empty(B, H, n, CHUNK, CHUNK, dtype=torch.bfloat16, device=dev)
         s_final = torch.empty(B, H, d, d, dtype=torch.float32, device=dev)
-        st = _lib.status_word(dev).data_ptr()
-        _lib.check(L.ceo_efla_fwd(qn.data_ptr(), kn.data_ptr(), v_ptr, alpha.data_ptr(),
-                                  _lib.ptr(s0), w.data_ptr(), up.data_ptr(), states.data_ptr(),
-                                  xinv.data_ptr(),
-                                  o.data_ptr(), s_final.data_ptr(), _lib.ptr(resets), B, T, H, d,
-                                  hd, hd, N, st,
-                                  _lib.stream()), "ceo_efla_fwd")
+        _fwd(qn.data_ptr(), kn.data_ptr(), v_ptr, alpha, s0, w, up, states, xinv, o, s_final,
+             resets, B, T, H, d, hd, hd, N)
         ctx.save_for_backward(proj, beta, qn, kn, rq, rk, alpha, w, up, states, xinv)
         ctx.cfg = (P, H, d, normalize, s0 is not None)
         return o, s_final
