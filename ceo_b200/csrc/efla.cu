@@ -1272,7 +1272,8 @@ efla_prep_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
                      const float* __restrict__ beta, int beta_scalar, bf16* __restrict__ qn,
                      bf16* __restrict__ kn, float* __restrict__ rq, float* __restrict__ rk,
                      float* __restrict__ alpha, long long rows, int H, long long qs, long long ks,
-                     int normalize) {
+                     int normalize, const bf16* __restrict__ logits, long long ls,
+                     float* __restrict__ beta_out) {
   constexpr int LPR = D / 8, RPW = 32 / LPR, U = 4;
   const int lane = threadIdx.x & 31, sub = lane % LPR, rw = lane / LPR;
   const unsigned wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1280,11 +1281,13 @@ efla_prep_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
   const unsigned total = static_cast<unsigned>(rows * H);
   for (unsigned id0 = wid * (RPW * U); id0 < total; id0 += nw * (RPW * U)) {
     uint4 qp[U], kp[U];
+    float bl[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const unsigned id = id0 + u * RPW + rw;
       const unsigned idc = id < total ? id : 0;
       const unsigned tok = idc / static_cast<unsigned>(H), h = idc - tok * H;
+      bl[u] = logits ? __bfloat162float(logits[tok * ls + h]) : beta_scalar ? beta[0] : beta[idc];
       qp[u] = *reinterpret_cast<const uint4*>(q + tok * qs + h * D + sub * 8);
       kp[u] = *reinterpret_cast<const uint4*>(k + tok * ks + h * D + sub * 8);
     }
@@ -1313,7 +1316,11 @@ efla_prep_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
       *reinterpret_cast<uint4*>(qn + static_cast<long long>(id) * D + sub * 8) = pack8(qv);
       *reinterpret_cast<uint4*>(kn + static_cast<long long>(id) * D + sub * 8) = pack8(kv);
       if (sub == 0) {
-        const float b = beta_scalar ? beta[0] : beta[id];
+        float b = bl[u];
+        if (logits) {
+          b = 1.f / (1.f + __expf(-b));
+          if (beta_out) beta_out[id] = b;
+        }
         rq[id] = iq;
         rk[id] = ik;
         alpha[id] = normalize ? -expm1f(-b) : efla_coeff(b, sk);
@@ -1332,7 +1339,8 @@ efla_prep_bwd_kernel(const bf16* __restrict__ dqn, const bf16* __restrict__ dkn,
                      const float* __restrict__ beta, int beta_scalar,
                      const float* __restrict__ dalpha, bf16* __restrict__ dq,
                      bf16* __restrict__ dk, float* __restrict__ dbeta, long long rows, int H,
-                     long long dqs, long long dks, int normalize) {
+                     long long dqs, long long dks, int normalize, bf16* __restrict__ dlogits,
+                     long long dls, int pad) {
   constexpr int LPR = D / 8, RPW = 32 / LPR, U = 2;
   const int lane = threadIdx.x & 31, sub = lane % LPR, rw = lane / LPR;
   const unsigned wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1402,7 +1410,14 @@ efla_prep_bwd_kernel(const bf16* __restrict__ dqn, const bf16* __restrict__ dkn,
       const unsigned tok = id / static_cast<unsigned>(H), h = id - tok * H;
       *reinterpret_cast<uint4*>(dq + tok * dqs + h * D + sub * 8) = pack8(oq);
       *reinterpret_cast<uint4*>(dk + tok * dks + h * D + sub * 8) = pack8(ok);
-      if (sub == 0) dbeta[id] = db;
+      if (dlogits) {
+        // beta = sigmoid(logit); the projection's padding columns get a zero gradient
+        if (sub == 0) dlogits[tok * dls + h] = __float2bfloat16(db * b * (1.f - b));
+        if (h == H - 1)
+          for (int c = sub; c < pad; c += LPR) dlogits[tok * dls + H + c] = __float2bfloat16(0.f);
+      } else if (sub == 0) {
+        dbeta[id] = db;
+      }
     }
   }
 }
@@ -1719,26 +1734,60 @@ extern "C" int ceo_efla_bwd(const void* q, const void* k, const void* v, const f
   return 0;
 }
 
-extern "C" int ceo_efla_prep_fwd(const void* q, const void* k, const float* beta, int beta_scalar,
-                                 void* qn, void* kn, float* rq, float* rk, float* alpha,
-                                 long long rows, int H, int D, long long q_stride,
-                                 long long k_stride, int normalize, cudaStream_t stream) {
+static int prep_fwd_run(const void* q, const void* k, const float* beta, int beta_scalar, void* qn,
+                        void* kn, float* rq, float* rk, float* alpha, long long rows, int H, int D,
+                        long long q_stride, long long k_stride, int normalize, const void* logits,
+                        long long logit_stride, float* beta_out, cudaStream_t stream) {
   if (rows <= 0 || H <= 0 || (D != 64 && D != 128) || rows * H >= (1LL << 31)) return -5;
   if (((q_stride | k_stride) & 7) ||
       ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
         reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn)) & 15))
     return -2;  // rows move as 16-byte accesses
   const int grid = grid_for(rows * H, 8 * 4 * (D == 64 ? 4 : 2), 148 * 4);  // one resident wave
-  if (D == 64)
-    efla_prep_fwd_kernel<64><<<grid, 256, 0, stream>>>(
-        static_cast<const bf16*>(q), static_cast<const bf16*>(k), beta, beta_scalar,
-        static_cast<bf16*>(qn), static_cast<bf16*>(kn), rq, rk, alpha, rows, H, q_stride, k_stride,
-        normalize);
-  else
-    efla_prep_fwd_kernel<128><<<grid, 256, 0, stream>>>(
-        static_cast<const bf16*>(q), static_cast<const bf16*>(k), beta, beta_scalar,
-        static_cast<bf16*>(qn), static_cast<bf16*>(kn), rq, rk, alpha, rows, H, q_stride, k_stride,
-        normalize);
+  auto kern = D == 64 ? efla_prep_fwd_kernel<64> : efla_prep_fwd_kernel<128>;
+  kern<<<grid, 256, 0, stream>>>(static_cast<const bf16*>(q), static_cast<const bf16*>(k), beta,
+                                 beta_scalar, static_cast<bf16*>(qn), static_cast<bf16*>(kn), rq,
+                                 rk, alpha, rows, H, q_stride, k_stride, normalize,
+                                 static_cast<const bf16*>(logits), logit_stride, beta_out);
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int ceo_efla_prep_fwd(const void* q, const void* k, const float* beta, int beta_scalar,
+                                 void* qn, void* kn, float* rq, float* rk, float* alpha,
+                                 long long rows, int H, int D, long long q_stride,
+                                 long long k_stride, int normalize, cudaStream_t stream) {
+  return prep_fwd_run(q, k, beta, beta_scalar, qn, kn, rq, rk, alpha, rows, H, D, q_stride,
+                      k_stride, normalize, nullptr, 0, nullptr, stream);
+}
+
+extern "C" int ceo_efla_prep_fwd_logits(const void* q, const void* k, const void* logits,
+                                        long long logit_stride, float* beta, void* qn, void* kn,
+                                        float* rq, float* rk, float* alpha, long long rows, int H,
+                                        int D, long long q_stride, long long k_stride,
+                                        int normalize, cudaStream_t stream) {
+  if (!logits) return -5;
+  return prep_fwd_run(q, k, nullptr, 0, qn, kn, rq, rk, alpha, rows, H, D, q_stride, k_stride,
+                      normalize, logits, logit_stride, beta, stream);
+}
+
+static int prep_bwd_run(const void* dqn, const void* dkn, const void* qn, const void* kn,
+                        const float* rq, const float* rk, const float* beta, int beta_scalar,
+                        const float* dalpha, void* dq, void* dk, float* dbeta, long long rows,
+                        int H, int D, long long dq_stride, long long dk_stride, int normalize,
+                        void* dlogits, long long dlogit_stride, int pad, cudaStream_t stream) {
+  if (rows <= 0 || H <= 0 || (D != 64 && D != 128) || rows * H >= (1LL << 31)) return -5;
+  if (((dq_stride | dk_stride) & 7) ||
+      ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
+        reinterpret_cast<uintptr_t>(dqn) | reinterpret_cast<uintptr_t>(dkn) |
+        reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn)) & 15))
+    return -2;  // rows move as 16-byte accesses
+  const int grid = grid_for(rows * H, 8 * 2 * (D == 64 ? 4 : 2), 148 * 3);  // one resident wave
+  auto kern = D == 64 ? efla_prep_bwd_kernel<64> : efla_prep_bwd_kernel<128>;
+  kern<<<grid, 256, 0, stream>>>(static_cast<const bf16*>(dqn), static_cast<const bf16*>(dkn),
+                                 static_cast<const bf16*>(qn), static_cast<const bf16*>(kn), rq, rk,
+                                 beta, beta_scalar, dalpha, static_cast<bf16*>(dq),
+                                 static_cast<bf16*>(dk), dbeta, rows, H, dq_stride, dk_stride,
+                                 normalize, static_cast<bf16*>(dlogits), dlogit_stride, pad);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -1747,24 +1796,19 @@ extern "C" int ceo_efla_prep_bwd(const void* dqn, const void* dkn, const void* q
                                  int beta_scalar, const float* dalpha, void* dq, void* dk,
                                  float* dbeta, long long rows, int H, int D, long long dq_stride,
                                  long long dk_stride, int normalize, cudaStream_t stream) {
-  if (rows <= 0 || H <= 0 || (D != 64 && D != 128) || rows * H >= (1LL << 31)) return -5;
-  if (((dq_stride | dk_stride) & 7) ||
-      ((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) |
-        reinterpret_cast<uintptr_t>(dqn) | reinterpret_cast<uintptr_t>(dkn) |
-        reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn)) & 15))
-    return -2;  // rows move as 16-byte accesses
-  const int grid = grid_for(rows * H, 8 * 2 * (D == 64 ? 4 : 2), 148 * 3);  // one resident wave
-  if (D == 64)
-    efla_prep_bwd_kernel<64><<<grid, 256, 0, stream>>>(
-        static_cast<const bf16*>(dqn), static_cast<const bf16*>(dkn), static_cast<const bf16*>(qn),
-        static_cast<const bf16*>(kn), rq, rk, beta, beta_scalar, dalpha, static_cast<bf16*>(dq),
-        static_cast<bf16*>(dk), dbeta, rows, H, dq_stride, dk_stride, normalize);
-  else
-    efla_prep_bwd_kernel<128><<<grid, 256, 0, stream>>>(
-        static_cast<const bf16*>(dqn), static_cast<const bf16*>(dkn), static_cast<const bf16*>(qn),
-        static_cast<const bf16*>(kn), rq, rk, beta, beta_scalar, dalpha, static_cast<bf16*>(dq),
-        static_cast<bf16*>(dk), dbeta, rows, H, dq_stride, dk_stride, normalize);
-  return static_cast<int>(cudaGetLastError());
+  return prep_bwd_run(dqn, dkn, qn, kn, rq, rk, beta, beta_scalar, dalpha, dq, dk, dbeta, rows, H,
+                      D, dq_stride, dk_stride, normalize, nullptr, 0, 0, stream);
+}
+
+extern "C" int ceo_efla_prep_bwd_logits(const void* dqn, const void* dkn, const void* qn,
+                                        const void* kn, const float* rq, const float* rk,
+                                        const float* beta, const float* dalpha, void* dq, void* dk,
+                                        void* dlogits, long long dlogit_stride, int pad,
+                                        long long rows, int H, int D, long long dq_stride,
+                                        long long dk_stride, int normalize, cudaStream_t stream) {
+  if (!dlogits || pad < 0 || dlogit_stride < H + pad) return -5;
+  return prep_bwd_run(dqn, dkn, qn, kn, rq, rk, beta, 0, dalpha, dq, dk, nullptr, rows, H, D,
+                      dq_stride, dk_stride, normalize, dlogits, dlogit_stride, pad, stream);
 }
 
 // ---------------------------------------------------------------------------------------

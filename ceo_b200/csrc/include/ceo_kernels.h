@@ -91,6 +91,21 @@ int ceo_efla_prep_bwd(const void* dqn, const void* dkn, const void* qn, const vo
                       int D, long long dq_stride, long long dk_stride, int normalize,
                       cudaStream_t stream);
 
+/* The same with per-token beta = sigmoid(logit), logits bf16 [rows][H] with a row stride (columns
+ * of the projection); forward also returns beta (fp32 (rows*H), may be NULL), backward writes
+ * the logits' gradient (bf16) and zeroes the `pad` columns behind them. */
+int ceo_efla_prep_fwd_logits(const void* q, const void* k, const void* logits,
+                             long long logit_stride, float* beta, void* qn, void* kn, float* rq,
+                             float* rk, float* alpha, long long rows, int H, int D,
+                             long long q_stride, long long k_stride, int normalize,
+                             cudaStream_t stream);
+int ceo_efla_prep_bwd_logits(const void* dqn, const void* dkn, const void* qn, const void* kn,
+                             const float* rq, const float* rk, const float* beta,
+                             const float* dalpha, void* dq, void* dk, void* dlogits,
+                             long long dlogit_stride, int pad, long long rows, int H, int D,
+                             long long dq_stride, long long dk_stride, int normalize,
+                             cudaStream_t stream);
+
 /* ---- token-by-token inference ------------------------------------------------
  * T tokens of each of B sequences (T = 1, or B = 1; B * T <= 128) through every block, states
  * updated in place; logits (fp32 [B][vocab], may be NULL) of each sequence's last token.

@@ -287,17 +287,17 @@ class _EflaProjFn(torch.autograd.Function):
         base = proj.data_ptr()
         q_ptr, k_ptr = base, base + (hd * esz if P == 3 else 0)
         v_ptr = base + (P - 1) * hd * esz
-        beta = torch.sigmoid(proj[..., P * hd:P * hd + H].float()).contiguous()
         L = _lib.lib()
         qn = torch.empty(B, T, H, d, dtype=torch.bfloat16, device=dev)
         kn = torch.empty_like(qn) if P == 3 else qn
         rq = torch.empty(B, T, H, dtype=torch.float32, device=dev)
         rk = torch.empty_like(rq)
         alpha = torch.empty_like(rq)
-        _lib.check(L.ceo_efla_prep_fwd(q_ptr, k_ptr, beta.data_ptr(), 0, qn.data_ptr(),
-                                       kn.data_ptr(), rq.data_ptr(), rk.data_ptr(),
-                                       alpha.data_ptr(), B * T, H, d, N, N, int(normalize),
-                                       _lib.stream()), "ceo_efla_prep_fwd")
+        beta = torch.empty_like(rq)
+        _lib.check(L.ceo_efla_prep_fwd_logits(
+            q_ptr, k_ptr, base + P * hd * esz, N, beta.data_ptr(), qn.data_ptr(), kn.data_ptr(),
+            rq.data_ptr(), rk.data_ptr(), alpha.data_ptr(), B * T, H, d, N, N, int(normalize),
+            _lib.stream()), "ceo_efla_prep_fwd_logits")
         w = torch.empty(B, T, H, d, dtype=torch.bfloat16, device=dev)
         up = torch.empty_like(w)
         o = torch.empty_like(w)
@@ -341,20 +341,16 @@ class _EflaProjFn(torch.autograd.Function):
                                   dalpha.data_ptr(), ds0.data_ptr(), _lib.ptr(ctx.resets), B, T, H,
                                   d, hd, hd, N, hd, hd,
                                   N, st, _lib.stream()), "ceo_efla_bwd")
-        dbeta = torch.empty(B, T, H, dtype=torch.float32, device=dev)
         if P == 3:
             dq_ptr, dk_ptr, dq_stride = dbase, dbase + hd * esz, N
         else:
             dkn.add_(dqn)
             dq_ptr, dk_ptr, dq_stride = dloc.data_ptr(), dbase, hd
-        _lib.check(L.ceo_efla_prep_bwd(dqn.data_ptr(), dkn.data_ptr(), qn.data_ptr(),
-                                       kn.data_ptr(), rq.data_ptr(), rk.data_ptr(),
-                                       beta.data_ptr(), 0, dalpha.data_ptr(), dq_ptr, dk_ptr,
-                                       dbeta.data_ptr(), B * T, H, d, dq_stride, N, int(normalize),
-                                       _lib.stream()), "ceo_efla_prep_bwd")
-        tail = dproj[..., P * hd:]
-        tail.zero_()
-        tail[..., :H].copy_(dbeta * beta * (1.0 - beta))
+        _lib.check(L.ceo_efla_prep_bwd_logits(
+            dqn.data_ptr(), dkn.data_ptr(), qn.data_ptr(), kn.data_ptr(), rq.data_ptr(),
+            rk.data_ptr(), beta.data_ptr(), dalpha.data_ptr(), dq_ptr, dk_ptr,
+            dbase + P * hd * esz, N, N - P * hd - H, B * T, H, d, dq_stride, N, int(normalize),
+            _lib.stream()), "ceo_efla_prep_bwd_logits")
         return dproj, None, None, None, None, (ds0 if has_s0 else None), None
 
 
