@@ -58,6 +58,7 @@ struct GemmParams {
   int out_f32;     // 1: C is fp32, 0: C is bf16
   int accumulate;  // C = alpha*acc + C
   float alpha;
+  float res_scale;  // C = alpha * acc + res_scale * residual
   // 8-bit float operands (K-major only): element formats (0 e4m3, 1 e5m2) and the device-side
   // quantisation scales; the epilogue multiplies by alpha / (scale_a * scale_b)
   int fp8_a, fp8_b;
@@ -838,8 +839,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                   const float2 x = __bfloat1622float2(h[j]);
-                  f[2 * j] += x.x;
-                  f[2 * j + 1] += x.y;
+                  f[2 * j] += p.res_scale * x.x;
+                  f[2 * j + 1] += p.res_scale * x.y;
                 }
               }
               uint4 o;
@@ -925,13 +926,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 float2 x = __bfloat1622float2(h[j]);
-                f[q * 8 + 2 * j] += x.x;
-                f[q * 8 + 2 * j + 1] += x.y;
+                f[q * 8 + 2 * j] += p.res_scale * x.x;
+                f[q * 8 + 2 * j + 1] += p.res_scale * x.y;
               }
             }
           } else {
             for (int j = 0; j < 32; ++j)
-              if (n + j < p.N) f[j] += __bfloat162float(rrow[n + j]);
+              if (n + j < p.N) f[j] += p.res_scale * __bfloat162float(rrow[n + j]);
           }
         }
         if (p.out_f32) {
@@ -1127,6 +1128,7 @@ struct EpiDesc {
   int mode = 0;
   void* aux = nullptr;
   long long ld_aux = 0;
+  float res_scale = 1.f;  // of the residual term
 };
 
 // Host-side description of the collective fused into a GEMM launch (see GemmParams).
@@ -1203,6 +1205,7 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   p.out_f32 = out_f32;
   p.accumulate = accumulate;
   p.alpha = alpha;
+  p.res_scale = epi.res_scale;
   p.fp8_a = f8.kind_a;
   p.fp8_b = f8.kind_b;
   p.scale_a = f8.scale_a;
@@ -1229,7 +1232,7 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   // row, 2.4 GB of weights) take 0.97 ms one after the other, and 0.96 ms the whole step when
   // chained (decode.cu); it was 12 ms.
   if (fz.kind == 0 && !f8.on && !a_mn_major && !b_mn_major && batch == 1 && !accumulate && !bias &&
-      max_ctas <= 0 && M <= 128 && epi.mode != 2) {
+      max_ctas <= 0 && M <= 128 && epi.mode != 2 && epi.res_scale == 1.f) {
     SkinnyArgs g = {};
     g.A = A; g.W = B; g.C = C; g.residual = residual; g.act = epi.mode == 1 ? epi.aux : nullptr;
     g.lda = lda; g.ldw = ldb; g.ldc = ldc; g.ldr = ldr; g.ldact = epi.ld_aux;
@@ -1348,6 +1351,21 @@ extern "C" int ceo_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   return gemm_run(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, batch, batch_stride_a,
                   batch_stride_b, batch_stride_c, out_f32, accumulate, alpha, bias, residual, ldr,
                   batch_stride_r, status, max_ctas, fz, stream);
+}
+
+// C[b] = alpha * A[b] B[b]^T + beta * R[b], all bf16 (the Newton-Schulz update).
+extern "C" int ceo_gemm_bf16_axpy(const void* A, const void* B, void* C, int M, int N, int K,
+                                  long long lda, long long ldb, long long ldc, int a_mn_major,
+                                  int b_mn_major, int batch, long long batch_stride_a,
+                                  long long batch_stride_b, long long batch_stride_c, float alpha,
+                                  float beta, const void* R, long long ldr,
+                                  long long batch_stride_r, int* status, cudaStream_t stream) {
+  FusedDesc fz;
+  EpiDesc epi;
+  epi.res_scale = beta;
+  return gemm_run(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, batch, batch_stride_a,
+                  batch_stride_b, batch_stride_c, 0, 0, alpha, nullptr, R, ldr, batch_stride_r,
+                  status, 0, fz, stream, 1, Fp8Desc(), epi);
 }
 
 // The bf16 GEMM with SwiGLU in its epilogue.  mode 1: C[M,N] = A B^T holds gate/up in

@@ -37,6 +37,13 @@ int ceo_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
                   const void* residual, long long ldr, long long batch_stride_r, int* status,
                   int max_ctas, cudaStream_t stream);
 
+/* C[b] = alpha * A[b] B[b]^T + beta * R[b]; everything bf16. */
+int ceo_gemm_bf16_axpy(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                       long long ldb, long long ldc, int a_mn_major, int b_mn_major, int batch,
+                       long long batch_stride_a, long long batch_stride_b,
+                       long long batch_stride_c, float alpha, float beta, const void* R,
+                       long long ldr, long long batch_stride_r, int* status, cudaStream_t stream);
+
 /* 1: weight-gradient GEMMs never split K (split-K accumulates with fp32 atomics, whose order
  * varies from run to run).  Default 0. */
 int ceo_set_deterministic(int on);
@@ -201,6 +208,15 @@ int ceo_ns_poly(void* g_bf16, const void* g2_bf16, int n, float a, float b, floa
                 cudaStream_t stream);
 /* gscale_ptr (optional): the device clip scale of the step; exactly 0 marks a step whose
  * gradient norm was not finite, which every update kernel above and this one then skip. */
+/* Up to 32 matrices of `numel` elements (a multiple of 4, 16-byte aligned, fp32 gradients) per
+ * call; m, grad, master, shadow are host arrays of device pointers.  prep: m = beta m + g, then
+ * y[i] (bf16, dense) = m_i / (|m_i|_F + eps); partial: fp32 [count][CEO_SUMSQ_MAX_BLOCKS]. */
+int ceo_muon_prep_multi(float* const* m, const float* const* grad, int count, long long numel,
+                        float beta, const float* gscale_ptr, float gscale, float* partial, void* y,
+                        float eps, cudaStream_t stream);
+int ceo_muon_apply_multi(float* const* master, const void* y, void* const* shadow, int count,
+                         long long numel, float lr, float weight_decay, float scale,
+                         const float* gscale_ptr, cudaStream_t stream);
 int ceo_muon_apply(float* master, const void* y_bf16, void* shadow_bf16, long long n, float lr,
                    float weight_decay, float scale, const float* gscale_ptr,
                    cudaStream_t stream);

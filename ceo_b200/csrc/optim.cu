@@ -208,6 +208,82 @@ __global__ void muon_apply_kernel(float* __restrict__ master, const bf16* __rest
   }
 }
 
+// The same three passes over up to 32 equally sized matrices per launch (blockIdx.y = matrix):
+// a model has some hundred Muon matrices, most of them too small to fill the chip or to hide a
+// launch.  16-byte accesses; bound by memory.
+constexpr int MUON_MAX = 32;
+struct MuonTable {
+  float* a[MUON_MAX];
+  const float* g[MUON_MAX];
+  bf16* s[MUON_MAX];
+};
+__global__ void __launch_bounds__(256)
+muon_momentum_multi_kernel(const MuonTable t, long long n4, float beta,
+                           const float* __restrict__ gscale_ptr, float gscale,
+                           float* __restrict__ partial) {
+  __shared__ float red[33];
+  const bool skip = step_skipped(gscale_ptr);
+  const float gs = gscale * (gscale_ptr ? *gscale_ptr : 1.f);
+  float4* m = reinterpret_cast<float4*>(t.a[blockIdx.y]);
+  const float4* g = reinterpret_cast<const float4*>(t.g[blockIdx.y]);
+  float s = 0.f;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n4; i += gridDim.x * 256LL) {
+    float4 v = m[i];
+    if (!skip) {
+      const float4 x = g[i];
+      v.x = beta * v.x + x.x * gs;
+      v.y = beta * v.y + x.y * gs;
+      v.z = beta * v.z + x.z * gs;
+      v.w = beta * v.w + x.w * gs;
+      m[i] = v;
+    }
+    s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+  }
+  s = block_reduce_sum(s, red);
+  if (threadIdx.x == 0) partial[blockIdx.y * CEO_SUMSQ_MAX_BLOCKS + blockIdx.x] = s;
+}
+__global__ void __launch_bounds__(256)
+muon_normalize_multi_kernel(const MuonTable t, long long n4, const float* __restrict__ partial,
+                            int nblk, bf16* __restrict__ y, float eps) {
+  __shared__ float red[33];
+  float s = 0.f;
+  for (int i = threadIdx.x; i < nblk; i += 256) s += partial[blockIdx.y * CEO_SUMSQ_MAX_BLOCKS + i];
+  const float inv = 1.f / (sqrtf(block_reduce_sum(s, red)) + eps);
+  const float4* m = reinterpret_cast<const float4*>(t.a[blockIdx.y]);
+  uint2* o = reinterpret_cast<uint2*>(y) + blockIdx.y * n4;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n4; i += gridDim.x * 256LL) {
+    const float4 v = m[i];
+    uint2 u;
+    *reinterpret_cast<bf162*>(&u.x) = __floats2bfloat162_rn(v.x * inv, v.y * inv);
+    *reinterpret_cast<bf162*>(&u.y) = __floats2bfloat162_rn(v.z * inv, v.w * inv);
+    o[i] = u;
+  }
+}
+__global__ void __launch_bounds__(256)
+muon_apply_multi_kernel(const MuonTable t, long long n4, const bf16* __restrict__ y, float lr,
+                        float wd, float scale, const float* __restrict__ gscale_ptr) {
+  if (step_skipped(gscale_ptr)) return;
+  float4* master = reinterpret_cast<float4*>(t.a[blockIdx.y]);
+  uint2* shadow = reinterpret_cast<uint2*>(t.s[blockIdx.y]);
+  const uint2* yy = reinterpret_cast<const uint2*>(y) + blockIdx.y * n4;
+  const float keep = 1.f - lr * wd, f = lr * scale;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n4; i += gridDim.x * 256LL) {
+    float4 p = master[i];
+    const uint2 u = yy[i];
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const bf162*>(&u.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const bf162*>(&u.y));
+    p.x = p.x * keep - f * a.x;
+    p.y = p.y * keep - f * a.y;
+    p.z = p.z * keep - f * b.x;
+    p.w = p.w * keep - f * b.y;
+    master[i] = p;
+    uint2 o;
+    *reinterpret_cast<bf162*>(&o.x) = __floats2bfloat162_rn(p.x, p.y);
+    *reinterpret_cast<bf162*>(&o.y) = __floats2bfloat162_rn(p.z, p.w);
+    shadow[i] = o;
+  }
+}
+
 // float4-vectorised variants for fp32 gradients (the flat main_grad buffer): 16-byte loads
 // and stores on every stream, 8-byte stores for the bf16 shadow.
 __global__ void __launch_bounds__(256)
@@ -427,5 +503,51 @@ extern "C" int ceo_muon_apply(float* master, const void* y_bf16, void* shadow_bf
   muon_apply_kernel<<<grid_for(n, 256 * 4, OPT_GRID_CAP), 256, 0, stream>>>(
       master, static_cast<const bf16*>(y_bf16), static_cast<bf16*>(shadow_bf16), n, lr,
       weight_decay, scale, gscale_ptr);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// CTAs per matrix: eight per SM over the whole table, none with less than 4 K elements.
+static int muon_multi_grid(int count, long long n4) {
+  long long g = 148 * 8 / count, most = (n4 + 1023) / 1024;
+  if (g > most) g = most;
+  return static_cast<int>(g < 1 ? 1 : g > CEO_SUMSQ_MAX_BLOCKS ? CEO_SUMSQ_MAX_BLOCKS : g);
+}
+
+extern "C" int ceo_muon_prep_multi(float* const* m, const float* const* grad, int count,
+                                   long long numel, float beta, const float* gscale_ptr,
+                                   float gscale, float* partial, void* y, float eps,
+                                   cudaStream_t stream) {
+  if (count < 1 || count > MUON_MAX || numel <= 0 || (numel & 3)) return -5;
+  MuonTable t = {};
+  uintptr_t al = reinterpret_cast<uintptr_t>(y);
+  for (int i = 0; i < count; ++i) {
+    t.a[i] = m[i];
+    t.g[i] = grad[i];
+    al |= reinterpret_cast<uintptr_t>(m[i]) | reinterpret_cast<uintptr_t>(grad[i]);
+  }
+  if (al & 15) return -2;
+  const long long n4 = numel / 4;
+  const dim3 g(muon_multi_grid(count, n4), count);
+  muon_momentum_multi_kernel<<<g, 256, 0, stream>>>(t, n4, beta, gscale_ptr, gscale, partial);
+  muon_normalize_multi_kernel<<<g, 256, 0, stream>>>(t, n4, partial, g.x, static_cast<bf16*>(y), eps);
+  return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int ceo_muon_apply_multi(float* const* master, const void* y, void* const* shadow,
+                                    int count, long long numel, float lr, float weight_decay,
+                                    float scale, const float* gscale_ptr, cudaStream_t stream) {
+  if (count < 1 || count > MUON_MAX || numel <= 0 || (numel & 3)) return -5;
+  MuonTable t = {};
+  uintptr_t al = reinterpret_cast<uintptr_t>(y), al8 = 0;
+  for (int i = 0; i < count; ++i) {
+    t.a[i] = master[i];
+    t.s[i] = static_cast<bf16*>(shadow[i]);
+    al |= reinterpret_cast<uintptr_t>(master[i]);
+    al8 |= reinterpret_cast<uintptr_t>(shadow[i]);
+  }
+  if ((al & 15) || (al8 & 7)) return -2;
+  const long long n4 = numel / 4;
+  muon_apply_multi_kernel<<<dim3(muon_multi_grid(count, n4), count), 256, 0, stream>>>(
+      t, n4, static_cast<const bf16*>(y), lr, weight_decay, scale, gscale_ptr);
   return static_cast<int>(cudaGetLastError());
 }

@@ -28,8 +28,10 @@ def _as2d(t: torch.Tensor) -> torch.Tensor:
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None,
          accumulate: bool = False, alpha: float = 1.0, bias: torch.Tensor | None = None,
-         residual: torch.Tensor | None = None, max_ctas: int = 0) -> torch.Tensor:
-    """``out = alpha * A @ B^T (+ bias) (+ residual) (+ out if accumulate)``.
+         residual: torch.Tensor | None = None, max_ctas: int = 0,
+         residual_scale: float = 1.0) -> torch.Tensor:
+    """``out = alpha * A @ B^T (+ bias) (+ residual_scale * residual) (+ out if accumulate)``
+    (a scale other than one: bf16 output, no other term).
 
     ``a`` is ``(M, K)`` (or ``(K, M)`` when ``a_mn``); ``b`` is ``(N, K)`` (or ``(K, N)``
     when ``b_mn``).  A leading batch dimension on both makes it a batched GEMM.
@@ -59,7 +61,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if bias is not None:
             r = r + bias.float()
         if residual is not None:
-            r = r + residual.float()
+            r = r + residual_scale * residual.float()
         if out is not None:
             if accumulate:
                 r = r + out.float()
@@ -80,6 +82,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         assert residual.dtype == torch.bfloat16 and residual.stride(-1) == 1
     if bias is not None:
         assert bias.dtype == torch.float32 and bias.is_contiguous()
+    if residual_scale != 1.0:
+        assert residual is not None and bias is None and not accumulate and not out_f32 \
+            and max_ctas == 0
+        rc = _lib.lib().ceo_gemm_bf16_axpy(
+            a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K,
+            a2.stride(0), b2.stride(0), out.stride(-2), int(a_mn), int(b_mn), nb,
+            a.stride(0) if batched else 0, b.stride(0) if batched else 0,
+            out.stride(0) if batched else 0, float(alpha), float(residual_scale),
+            residual.data_ptr(), residual.stride(-2), residual.stride(0) if batched else 0,
+            _lib.status_word(a.device).data_ptr(), _lib.stream())
+        _lib.check(rc, "ceo_gemm_bf16_axpy")
+        return out
     rc = _lib.lib().ceo_gemm_bf16(
         a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K,
         a2.stride(0), b2.stride(0), out.stride(-2), int(a_mn), int(b_mn), nb,

@@ -12,6 +12,7 @@ scale stays on the device, Newton-Schulz products run on the tcgen05 GEMM.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import torch
@@ -237,32 +238,80 @@ class ShardedOptimizer:
             shadow.copy_(f.master[a:b])
 
     def _newton_schulz(self, y):
-        """y: (n, m) bf16, Frobenius-normalised.  Returns the orthogonalised matrix (bf16)."""
-        n, m = y.shape
+        """y: (n, m) or (batch, n, m) bf16, Frobenius-normalised matrices.  Returns the
+        orthogonalised matrices (bf16)."""
+        n, m = y.shape[-2:]
         small_left = n <= m
         L = _lib.lib()
         for _ in range(self.muon_iterations):
             a = gemm(y, y) if small_left else gemm(y, y, a_mn=True, b_mn=True)
-            k = a.shape[0]
             if self.muon_ns == "cubic":
-                _lib.check(L.ceo_ns_poly(a.data_ptr(), None, k, 1.5, -0.5, 0.0, _lib.stream()),
-                           "ceo_ns_poly")
-            else:
-                a2 = gemm(a, a)
-                _lib.check(L.ceo_ns_poly(a.data_ptr(), a2.data_ptr(), k, 3.4445, -4.7750, 2.0315,
-                                         _lib.stream()), "ceo_ns_poly")
+                # y <- (1.5 I - 0.5 a) y with the polynomial in the product's epilogue
+                y = gemm(a, y, b_mn=True, alpha=-0.5, residual=y, residual_scale=1.5) \
+                    if small_left else gemm(y, a, alpha=-0.5, residual=y, residual_scale=1.5)
+                continue
+            a2 = gemm(a, a)
+            for ai, a2i in zip(a, a2) if y.dim() == 3 else ((a, a2),):
+                _lib.check(L.ceo_ns_poly(ai.data_ptr(), a2i.data_ptr(), ai.shape[0], 3.4445,
+                                         -4.7750, 2.0315, _lib.stream()), "ceo_ns_poly")
             y = gemm(a, y, b_mn=True) if small_left else gemm(y, a)
         return y
+
+    def _muon_state_of(self, seg):
+        """Momentum and fp32 master of one Muon matrix, created on its first step."""
+        st = self._muon_state.get(seg.name)
+        if st is None:
+            f = self.flat
+            p = f.params[seg.offset:seg.offset + seg.numel]
+            st = {"momentum": torch.zeros(seg.numel, dtype=torch.float32, device=f.device),
+                  "master": p.float().clone()}
+            self._muon_state[seg.name] = st
+        return st
+
+    def _muon_group(self, segs, lr, gscale):
+        """Muon on equally shaped matrices together: the Newton-Schulz products become batched
+        GEMMs.  One 1024 x 1024 product is 32 tiles for 148 SMs; the 24 layers' are 768."""
+        f = self.flat
+        numel, k = segs[0].numel, len(segs)
+        st = [self._muon_state_of(s) for s in segs]
+        tab = lambda ptrs: (ctypes.c_void_p * k)(*ptrs)
+        L = _lib.lib()
+        y = torch.empty((k, *segs[0].shape), dtype=torch.bfloat16, device=f.device)
+        part = torch.empty(k * L.ceo_sumsq_blocks(1 << 40), dtype=torch.float32, device=f.device)
+        _lib.check(L.ceo_muon_prep_multi(
+            tab(s["momentum"].data_ptr() for s in st),
+            tab(f.grads.data_ptr() + 4 * s.offset for s in segs), k, numel, self.muon_momentum,
+            self._scale.data_ptr(), float(gscale), part.data_ptr(), y.data_ptr(), 1e-7,
+            _lib.stream()), "ceo_muon_prep_multi")
+        y = self._newton_schulz(y)
+        _lib.check(L.ceo_muon_apply_multi(
+            tab(s["master"].data_ptr() for s in st), y.data_ptr(),
+            tab(f.params.data_ptr() + 2 * s.offset for s in segs), k, numel, float(lr), 0.0, 1.0,
+            self._scale.data_ptr(), _lib.stream()), "ceo_muon_apply_multi")
+
+    def _muon_update(self, segs, lr, gscale):
+        """Muon on the matrices this rank owns."""
+        f = self.flat
+        groups = {}
+        for s in segs:
+            groups.setdefault(s.shape, []).append(s)
+        for shape, g in groups.items():
+            if not (self.cuda and f.param_dtype == torch.bfloat16
+                    and f.grads.dtype == torch.float32 and shape[0] * shape[1] % 4 == 0):
+                for s in g:
+                    self._muon_matrix(s, f.grads, lr, gscale)
+                continue
+            # at most 32 matrices (the kernels' pointer table) and 2^28 elements (512 MB of bf16
+            # per copy) at a time: by then every product fills the chip many times over
+            k = max(1, min(32, (1 << 28) // (shape[0] * shape[1])))
+            for i in range(0, len(g), k):
+                self._muon_group(g[i:i + k], lr, gscale)
 
     def _muon_matrix(self, seg, g_full, lr, gscale):
         """Muon on one whole matrix (this rank owns it).  g_full: the full fp32 grad buffer."""
         f = self.flat
-        st = self._muon_state.get(seg.name)
+        st = self._muon_state_of(seg)
         p = f.params[seg.offset:seg.offset + seg.numel]
-        if st is None:
-            st = {"momentum": torch.zeros(seg.numel, dtype=torch.float32, device=f.device),
-                  "master": p.float().clone()}
-            self._muon_state[seg.name] = st
         g = g_full[seg.offset:seg.offset + seg.numel]
         if self.cuda and f.param_dtype == torch.bfloat16:
             L = _lib.lib()
@@ -361,9 +410,7 @@ class ShardedOptimizer:
                     self._lion_range(gs, a, b, seg.decay, lr, grad_scale)
             if self._world() > 1:
                 self.comm.all_gather(f.params, f.lo, f.hi)
-            for i, seg in enumerate(self._matrix_segs):
-                if i % self._world() == f.rank:
-                    self._muon_matrix(seg, f.grads, lr, grad_scale)
+            self._muon_update(self._matrix_segs[f.rank::self._world()], lr, grad_scale)
             if self._world() > 1:
                 self.comm.broadcast_segments(f, self._matrix_segs)
         else:
