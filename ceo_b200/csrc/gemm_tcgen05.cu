@@ -102,7 +102,7 @@ struct GemmParams {
   long long rs_ldo;
   int rank, world;
   // SwiGLU fused into the epilogue (bf16 C, K-major or MN-major operands alike):
-  //   1  C holds gate/up in INTERLEAVED columns (2j = gate_j, 2j+1 = up_j); besides C the
+  //   1  C (may be null) holds gate/up in INTERLEAVED columns (2j = gate_j, 2j+1 = up_j); besides C the
   //      epilogue writes act[:, j] = silu(gate_j) * up_j into aux (M x N/2, ld_aux)
   //   2  the accumulator is d(act) (M x N); aux is the saved interleaved gate/up (M x 2N,
   //      ld_aux); C receives the interleaved d(gate/up) (M x 2N, ldc) and d(act) never
@@ -701,7 +701,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           for (int i = 0; i < 8; ++i) {
             const int rl = i * 4 + (lane >> 3);
             const uint4 o = *reinterpret_cast<const uint4*>(sb + rl * EPI_ROW_BYTES + (lane & 7) * 16);
-            if (row0 + rl < p.M && ncol < p.N)
+            if (cbase && row0 + rl < p.M && ncol < p.N)
               *reinterpret_cast<uint4*>(gbase + static_cast<long long>(rl) * p.ldc + ncol) = o;
           }
           const int acol = (n0 + c2 * 64) / 2 + (lane & 3) * 8;  // 32 act columns per chunk
@@ -1381,7 +1381,7 @@ extern "C" int ceo_gemm_bf16_swiglu(const void* A, const void* B, void* C, int M
   epi.mode = mode;
   epi.aux = aux;
   epi.ld_aux = ld_aux;
-  if (mode != 1 && mode != 2) return -5;
+  if ((mode != 1 && mode != 2) || (mode == 2 && !C)) return -5;
   return gemm_run(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, 1, 0, 0, 0, 0, 0, alpha,
                   nullptr, nullptr, 0, 0, status, 0, fz, stream, 1, Fp8Desc(), epi);
 }

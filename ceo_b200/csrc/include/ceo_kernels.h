@@ -127,6 +127,17 @@ int ceo_decode_tokens(const long long* ids, const void* table, long long vocab,
                       int n_proj, int F, int normalize, float eps, int* status,
                       cudaStream_t stream);
 
+/* Whole sequences without a backward pass: ids (B,T), T % 64 == 0 -> out = the final norm's rows
+ * (bf16 (B*T, hidden)); layers: host array of n_layers x 9 device pointers {ln1.weight, w_qkv,
+ * w_o, ln2.weight, w_up, w_down, scalar beta or NULL, s0 or NULL, s_final}, weights as for
+ * ceo_decode_tokens; resets as for ceo_efla_fwd.  ws: 256-byte aligned, the sum of its parts in
+ * the order taken (csrc/forward.cu), each rounded up to 256 bytes. */
+int ceo_forward_tokens(const long long* ids, const void* table, long long vocab,
+                       void* const* layers, int n_layers, const void* final_norm, void* out,
+                       void* ws, long long ws_bytes, const unsigned char* resets, int B, int T,
+                       int hidden, int H, int D, int P, int n_proj, int F, int normalize, float eps,
+                       int* status, cudaStream_t stream);
+
 /* ---- normalisation ---------------------------------------------------------- */
 int ceo_norm_bwd_blocks(int rows); /* rows of the partial scratch the bwd kernels need */
 int ceo_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* h_out,

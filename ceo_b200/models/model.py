@@ -255,6 +255,10 @@ class EflaLM(nn.Module):
         return self.embed_tokens if self.lm_head is None else self.lm_head
 
     def hidden(self, tokens, states=None, resets=None):
+        if tokens.is_cuda and not torch.is_grad_enabled():
+            out = decode_ops.forward_hidden(self, tokens, states, resets)
+            if out is not None:
+                return out
         h = K.embedding(tokens, self.embed_tokens)
         finals = []
         for i, blk in enumerate(self.blocks):

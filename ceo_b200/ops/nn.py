@@ -350,7 +350,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
     two gradient GEMMs of the chunk run before the next chunk's logits overwrite the buffer."""
 
     @staticmethod
-    def forward(ctx, x, weight, targets, label_smoothing, ignore_index, chunk_rows):
+    def forward(ctx, x, weight, targets, label_smoothing, ignore_index, chunk_rows, grads=True):
         D = x.shape[-1]
         x2 = x.reshape(-1, D)
         t = targets.reshape(-1).to(torch.int64).contiguous()
@@ -358,7 +358,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         n_valid = (t != ignore_index).sum().clamp(min=1).to(torch.float32)
         inv = (1.0 / n_valid).reshape(1)
         losses = torch.empty(rows, dtype=torch.float32, device=x.device)
-        need_grad = x.requires_grad or weight.requires_grad
+        need_grad = grads and (x.requires_grad or weight.requires_grad)
         dx = torch.empty_like(x2) if need_grad else None
         mg = getattr(weight, "main_grad", None)
         dw = None
@@ -399,7 +399,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         # gradients were computed with d(loss)=1; rescale if the caller scaled the loss
         gx = (dx * dloss.to(dx.dtype)).view(ctx.x_shape) if dx is not None else None
         gw = (dw * dloss).to(ctx.wdtype) if dw is not None else None
-        return gx, gw, None, None, None, None
+        return gx, gw, None, None, None, None, None
 
 
 def linear_cross_entropy(x, weight, targets, label_smoothing: float = 0.0,
@@ -410,8 +410,9 @@ def linear_cross_entropy(x, weight, targets, label_smoothing: float = 0.0,
     micro-batch scale into the optimizer's gradient scale instead)."""
     if not x.is_cuda:
         return ref.linear_cross_entropy(x, weight, targets, label_smoothing, ignore_index)
+    # grad mode is off inside a Function's forward: whether anybody will ask is known only here
     return _LinearCrossEntropyFn.apply(x, weight, targets, label_smoothing, ignore_index,
-                                       chunk_rows)
+                                       chunk_rows, torch.is_grad_enabled())
 
 
 def cross_entropy_rows(logits, targets, label_smoothing: float = 0.0, ignore_index: int = -100):
