@@ -273,6 +273,10 @@ int ceo_fp8_quantize_t(const void* x_bf16, void* q, void* qt, int rows, int cols
                        const float* scale, float* amax_out, int kind, cudaStream_t stream);
 int ceo_fp8_dequantize(const void* q, void* x_bf16, long long n, const float* scale, int kind,
                        cudaStream_t stream);
+/* up to 64 tensors: ptrs = host array of count x {history, cursor, amax, scale}, fp8_max = host
+ * array of count */
+int ceo_fp8_update_scales(void* const* ptrs, const float* fp8_max, int count, int hist_len,
+                          float margin_pow2, cudaStream_t stream);
 int ceo_fp8_update_scale(float* history, int hist_len, int* cursor, float* amax, float* scale,
                          float fp8_max, float margin_pow2, cudaStream_t stream);
 

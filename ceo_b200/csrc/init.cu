@@ -173,6 +173,30 @@ __global__ void fp8_update_scale_kernel(float* history, int hist_len, int* curso
   *amax = 0.f;
 }
 
+// The same for up to 64 tensors, one thread each (a model has some hundred scales and each
+// update alone is a launch).
+constexpr int FP8_TAB = 64;
+struct Fp8Table {
+  float* history[FP8_TAB];
+  int* cursor[FP8_TAB];
+  float* amax[FP8_TAB];
+  float* scale[FP8_TAB];
+  float fp8_max[FP8_TAB];
+};
+__global__ void fp8_update_scales_kernel(const Fp8Table t, int count, int hist_len,
+                                         float margin_pow2) {
+  const int i = threadIdx.x;
+  if (i >= count) return;
+  float* history = t.history[i];
+  const int cur = *t.cursor[i];
+  history[cur % hist_len] = *t.amax[i];
+  *t.cursor[i] = (cur + 1) % hist_len;
+  float m = 0.f;
+  for (int j = 0; j < hist_len; ++j) m = fmaxf(m, history[j]);
+  *t.scale[i] = (m > 0.f && isfinite(m)) ? t.fp8_max[i] / (m * margin_pow2) : 1.f;
+  *t.amax[i] = 0.f;
+}
+
 constexpr int GEN_CAP = 148 * 8;
 
 }  // namespace ceo
@@ -289,5 +313,20 @@ extern "C" int ceo_fp8_update_scale(float* history, int hist_len, int* cursor, f
   if (hist_len <= 0) return -5;
   fp8_update_scale_kernel<<<1, 1, 0, stream>>>(history, hist_len, cursor, amax, scale, fp8_max,
                                                margin_pow2);
+  return static_cast<int>(cudaGetLastError());
+}
+// ptrs: host array of count x 4 device pointers {history, cursor, amax, scale}, count <= 64.
+extern "C" int ceo_fp8_update_scales(void* const* ptrs, const float* fp8_max, int count,
+                                     int hist_len, float margin_pow2, cudaStream_t stream) {
+  if (hist_len <= 0 || count < 1 || count > FP8_TAB) return -5;
+  Fp8Table t = {};
+  for (int i = 0; i < count; ++i) {
+    t.history[i] = static_cast<float*>(ptrs[4 * i]);
+    t.cursor[i] = static_cast<int*>(ptrs[4 * i + 1]);
+    t.amax[i] = static_cast<float*>(ptrs[4 * i + 2]);
+    t.scale[i] = static_cast<float*>(ptrs[4 * i + 3]);
+    t.fp8_max[i] = fp8_max[i];
+  }
+  fp8_update_scales_kernel<<<1, FP8_TAB, 0, stream>>>(t, count, hist_len, margin_pow2);
   return static_cast<int>(cudaGetLastError());
 }

@@ -24,6 +24,8 @@ Without a GPU the same arithmetic runs through ``torch.float8_e4m3fn`` casts in 
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -192,7 +194,13 @@ class Fp8LinearState:
 
     def weight_q(self, weight: torch.Tensor) -> torch.Tensor:
         if self.wq is None or self.wq_step != self.recipe.step_id:
-            self.wq = quantize(weight.detach(), self.w_meta)
+            if self.recipe.dgrad and weight.requires_grad \
+                    and weight.shape[0] % 16 == 0 and weight.shape[1] % 16 == 0:
+                # the backward pass will want the transposed codes: one read gives both
+                self.wq, self.wtq = quantize_t(weight.detach(), self.w_meta)
+                self.wtq_step = self.recipe.step_id
+            else:
+                self.wq = quantize(weight.detach(), self.w_meta)
             self.wq_step = self.recipe.step_id
         return self.wq
 
@@ -200,6 +208,8 @@ class Fp8LinearState:
         """e4m3 codes of ``weight^T`` (in, out), on the scale of ``weight_q``."""
         if self.wtq is None or self.wtq_step != self.recipe.step_id:
             self.weight_q(weight)  # makes sure the weight's scale is calibrated
+            if self.wtq is not None and self.wtq_step == self.recipe.step_id:
+                return self.wtq
             self.wtq = _quantize_raw(transpose2d(weight.detach()), self.w_meta)
             self.wtq_step = self.recipe.step_id
         return self.wtq
@@ -221,13 +231,20 @@ class Fp8Recipe:
         return st
 
     def step(self) -> None:
-        for st in self.states:
-            if st.x_meta.calibrated:
-                st.x_meta.update()
-            if st.w_meta.calibrated:
-                st.w_meta.update()
-            if st.g_meta.calibrated:
-                st.g_meta.update()
+        metas = [m for st in self.states for m in (st.x_meta, st.w_meta, st.g_meta)
+                 if m.calibrated]
+        if metas and metas[0].scale.is_cuda:
+            for i in range(0, len(metas), 64):  # 64 tensors a launch
+                part = metas[i:i + 64]
+                ptrs = (ctypes.c_void_p * (4 * len(part)))(*(
+                    t.data_ptr() for m in part for t in (m.history, m.cursor, m.amax, m.scale)))
+                fmax = (ctypes.c_float * len(part))(*(_FMAX[m.kind] for m in part))
+                _lib.check(_lib.lib().ceo_fp8_update_scales(
+                    ptrs, fmax, len(part), self.history, 2.0 ** self.margin, _lib.stream()),
+                    "ceo_fp8_update_scales")
+        else:
+            for m in metas:
+                m.update()
         self.step_id += 1
 
     def invalidate(self) -> None:
