@@ -294,10 +294,24 @@ __device__ __forceinline__ bool ag_copy_all(const GemmParams& p, uint8_t* smem, 
   return ok;
 }
 
-template <int A_MN, int B_MN, int FP8 = 0>
+// TN: tile width, 256 or 128 (with six stages instead of four in the same shared memory).
+// PAIR: two CTAs of a cluster compute one 256 x 256 tile (cta_group::2).  Each holds its 128
+// rows of A and HALF of B's rows in shared memory and its 128 accumulator rows in TMEM; the
+// even CTA issues the MMAs for both.  Per CTA and k-block that is 32 KB instead of 48 KB through
+// L2 and shared memory, and six stages instead of four.  The collectives use single CTAs of 256.
+template <int A_MN, int B_MN, int FP8 = 0, int TN = 256, int PAIR = 0>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                          const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
+  constexpr int BN = TN;
+  constexpr int B_ROWS = PAIR ? TN / 2 : TN;  // rows of B in this CTA's stage
+  constexpr int STAGES = B_ROWS == 256 ? 4 : 6;
+  constexpr int STAGE_BYTES = A_STAGE_BYTES + B_ROWS * BK * 2;
+  constexpr int TM = PAIR ? 2 * BM : BM;      // rows of a tile
+  const int pair_rank = PAIR ? static_cast<int>(blockIdx.x & 1) : 0;
+  const int worker = static_cast<int>(blockIdx.x) >> PAIR, workers = static_cast<int>(gridDim.x) >> PAIR;
+  constexpr uint32_t TMEM_COLS = 2 * TN;
+  static_assert(STAGES * STAGE_BYTES == ceo::STAGES * ceo::STAGE_BYTES, "same ring");
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment: required by the 128B swizzle atom (8 rows x 128 B).
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -319,7 +333,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 4);
+      mbar_init(&tempty_bar[a], PAIR ? 8 : 4);  // the epilogue warps of both CTAs
     }
     if (p.ag_all)
       for (int i = 0; i < AG_RING; ++i) mbar_init(&bars[AG_RING_BAR + i], 1);
@@ -328,11 +342,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     tma_prefetch_desc(&tmB);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(tmem_slot, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -343,11 +363,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   // the first ag_ctas CTAs are helpers: they copy (all-gather) or reduce (reduce-scatter);
   // the others walk the output tiles
   const bool copy_cta = static_cast<int>(blockIdx.x) < p.ag_ctas;
-  const int tile_step = static_cast<int>(gridDim.x) - p.ag_ctas;
+  const int tile_step = workers - p.ag_ctas;
   // split-K: a work unit is (k-slice, tile); slices of one tile accumulate into C with atomics
   const int total_units = total_tiles * p.split_k;
   const int kb_per_split = (num_kb + p.split_k - 1) / p.split_k;
-  const int first_tile = copy_cta ? total_units : static_cast<int>(blockIdx.x) - p.ag_ctas;
+  const int first_tile = copy_cta ? total_units : worker - p.ag_ctas;
 
   if (p.rs_on && copy_cta) {
     // ------------------------------------------------ reduce-scatter: reducer CTA
@@ -371,8 +391,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
         const int r = tt - b * tiles_per_batch;
         int mb_, nb_;
         tile_coords(p, r, mb_, nb_);
-        const int m0 = mb_ * BM, n0 = nb_ * BN;
-        if (p.ag_operand) {
+        const int m0 = mb_ * TM + pair_rank * BM, n0 = nb_ * BN + pair_rank * B_ROWS;
+        if (!PAIR && p.ag_operand) {
           // rows pulled from a peer become loadable once the copy CTAs have published them
           const int row0 = p.ag_operand == 1 ? m0 : n0;
           const int rows = p.ag_operand == 1 ? p.M : p.N;
@@ -409,25 +429,60 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           uint8_t* sa = smem + s * STAGE_BYTES;
           uint8_t* sb = sa + A_STAGE_BYTES;
-          mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
           const int k0 = kb * BKE;
-          if (A_MN == 0) {
-            tma_load_3d(sa, &tmA, &full_bar[s], k0, m0, b);
-          } else if (p.a_4d) {
-            tma_load_4d(sa, &tmA, &full_bar[s], 0, k0, m0 / 64, b);
-          } else {
+          if (PAIR) {
+            // both CTAs' bytes count on the leader's barrier
+            if (pair_rank == 0) mbar_arrive_expect_tx(&full_bar[s], 2 * STAGE_BYTES);
+            const uint32_t lead = mapa_u32(smem_u32(&full_bar[s]), 0);
+            if (A_MN == 0) {
+              tma_load_3d_pair(sa, &tmA, lead, k0, m0, b);
+            } else if (p.a_4d) {
+              tma_load_4d_pair(sa, &tmA, lead, 0, k0, m0 / 64, b);
+            } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j)
-              tma_load_3d(sa + j * PANEL_BYTES, &tmA, &full_bar[s], m0 + j * 64, k0, b);
+              for (int j = 0; j < BM / 64; ++j)
+                tma_load_3d_pair(sa + j * PANEL_BYTES, &tmA, lead, m0 + j * 64, k0, b);
+            }
+            if (B_MN == 0) {
+              tma_load_3d_pair(sb, &tmB, lead, k0, n0, b);
+            } else if (p.b_4d) {
+              tma_load_4d_pair(sb, &tmB, lead, 0, k0, n0 / 64, b);
+            } else {
+#pragma unroll
+              for (int j = 0; j < B_ROWS / 64; ++j)
+                tma_load_3d_pair(sb + j * PANEL_BYTES, &tmB, lead, n0 + j * 64, k0, b);
+            }
+          } else {
+            mbar_arrive_expect_tx(&full_bar[s], STAGE_BYTES);
+            if (A_MN == 0) {
+              tma_load_3d(sa, &tmA, &full_bar[s], k0, m0, b);
+            } else if (p.a_4d) {
+              tma_load_4d(sa, &tmA, &full_bar[s], 0, k0, m0 / 64, b);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BM / 64; ++j)
+                tma_load_3d(sa + j * PANEL_BYTES, &tmA, &full_bar[s], m0 + j * 64, k0, b);
+            }
+            if (B_MN == 0) {
+              tma_load_3d(sb, &tmB, &full_bar[s], k0, n0, b);
+            } else if (p.b_4d) {
+              tma_load_4d(sb, &tmB, &full_bar[s], 0, k0, n0 / 64, b);
+            } else {
+#pragma unroll
+              for (int j = 0; j < BN / 64; ++j)
+                tma_load_3d(sb + j * PANEL_BYTES, &tmB, &full_bar[s], n0 + j * 64, k0, b);
+            }
           }
-          if (B_MN == 0) {
-            tma_load_3d(sb, &tmB, &full_bar[s], k0, n0, b);
-          } else if (p.b_4d) {
-            tma_load_4d(sb, &tmB, &full_bar[s], 0, k0, n0 / 64, b);
-          } else {
-#pragma unroll
-            for (int j = 0; j < BN / 64; ++j)
-              tma_load_3d(sb + j * PANEL_BYTES, &tmB, &full_bar[s], n0 + j * 64, k0, b);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
+        }
+      }
+      if (PAIR && ok) {
+        // the leader's last commits arrive on this CTA's barriers: stay until they have
+        for (int i = 0; i < STAGES; ++i) {
+          if (!mbar_wait(&empty_bar[s], ph ^ 1)) {
+            atomicCAS(p.status, 0, ST_PRODUCER);
+            ok = false;
+            break;
           }
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
@@ -527,9 +582,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = FP8 ? umma_idesc_f8(BM, BN, p.fp8_a, p.fp8_b)
-                                 : umma_idesc_bf16(BM, BN, A_MN, B_MN);
+    if (lane == 0 && pair_rank == 0) {
+      const uint32_t idesc = FP8 ? umma_idesc_f8(TM, BN, p.fp8_a, p.fp8_b)
+                                 : umma_idesc_bf16(TM, BN, A_MN, B_MN);
       const uint32_t smem0 = smem_u32(smem);
       const uint64_t adesc0 = A_MN ? umma_smem_desc(smem0, PANEL_BYTES, 1024)
                                    : umma_smem_desc(smem0, 16, 1024);
@@ -567,13 +622,23 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
             const uint64_t ad = ad0 + static_cast<uint64_t>(k) * ((A_MN ? 2048 : 32) >> 4);
             const uint64_t bd = bd0 + static_cast<uint64_t>(k) * ((B_MN ? 2048 : 32) >> 4);
             const uint32_t accf = (kb > kb0 || k != 0) ? 1u : 0u;
-            if (FP8) umma_f8(d_tmem, ad, bd, idesc, accf);
-            else umma_f16(d_tmem, ad, bd, idesc, accf);
+            if (PAIR) {
+              if (FP8) umma_f8_pair(d_tmem, ad, bd, idesc, accf);
+              else umma_f16_pair(d_tmem, ad, bd, idesc, accf);
+            } else {
+              if (FP8) umma_f8(d_tmem, ad, bd, idesc, accf);
+              else umma_f16(d_tmem, ad, bd, idesc, accf);
+            }
           }
-          umma_commit(&empty_bar[s]);  // frees the stage once these MMAs have read it
+          // frees the stage once these MMAs have read it
+          if (PAIR) umma_commit_pair(&empty_bar[s]);
+          else umma_commit(&empty_bar[s]);
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
-        if (ok) umma_commit(&tfull_bar[acc]);
+        if (ok) {
+          if (PAIR) umma_commit_pair(&tfull_bar[acc]);
+          else umma_commit(&tfull_bar[acc]);
+        }
       }
     }
   } else {
@@ -591,7 +656,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       const int r = tt - b * tiles_per_batch;
       int mb_, nb_;
       tile_coords(p, r, mb_, nb_);
-      const int m0 = mb_ * BM, n0 = nb_ * BN;
+      const int m0 = mb_ * TM + pair_rank * BM, n0 = nb_ * BN;
       if (!mbar_wait(&tfull_bar[acc], acc_ph)) {
         if (lane == 0) atomicCAS(p.status, 0, ST_EPILOGUE);
         ok = false;
@@ -862,14 +927,30 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
           }
           __syncwarp();
         }
-      } else if (p.out_f32 && !p.bias && !p.residual && p.split_k == 1 &&
-                 ((p.N | p.ldc) & 3) == 0) {
+      } else if (p.out_f32 && !p.bias && !p.residual && ((p.N | p.ldc) & 3) == 0) {
         // fp32 output (weight gradients, usually accumulating): 32 columns at a time through
-        // the same per-warp tile, so the read-modify-write of C moves whole 128-byte lines
+        // the same per-warp tile, so the read-modify-write of C (or, with k-slices, the vector
+        // reductions that replace it) moves whole 128-byte lines
+        const bool rmw = p.accumulate && p.split_k == 1;
         uint8_t* sb = smem + STAGES * STAGE_BYTES + 256 + quad * EPI_WARP_BYTES;
         const int row0 = m0 + quad * 32;
         float* gbase = reinterpret_cast<float*>(cbase) + static_cast<long long>(b) * p.batch_stride_c +
                        static_cast<long long>(row0) * p.ldc;
+        // what C held: a chunk's eight loads are requested together and one chunk ahead.  Behind
+        // the stores of the chunk before they would be one global round trip each, 64 a tile:
+        // the 1024 x 1024 gradient of 2176 tokens took 62 us that way and takes 33 us this way.
+        float4 old[8];
+        auto fetch_c = [&](int c) {
+          const int ncol = n0 + c * 32 + (lane & 7) * 4;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rl = i * 4 + (lane >> 3);
+            old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row0 + rl < p.M && ncol < p.N)
+              old[i] = *reinterpret_cast<const float4*>(gbase + static_cast<long long>(rl) * p.ldc + ncol);
+          }
+        };
+        if (rmw) fetch_c(0);
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
           uint32_t v[32];
@@ -883,18 +964,27 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
                             __uint_as_float(v[4 * q + 3]) * alpha);
           __syncwarp();
           const int ncol = n0 + c * 32 + (lane & 7) * 4;
+          float4 o[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const int rl = i * 4 + (lane >> 3);
-            float4 o = *reinterpret_cast<const float4*>(sb + rl * EPI_ROW_BYTES + (lane & 7) * 16);
-            if (row0 + rl < p.M && ncol < p.N) {
-              float4* dst = reinterpret_cast<float4*>(gbase + static_cast<long long>(rl) * p.ldc + ncol);
-              if (p.accumulate) {
-                const float4 old = *dst;
-                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-              }
-              *dst = o;
+            o[i] = *reinterpret_cast<const float4*>(sb + rl * EPI_ROW_BYTES + (lane & 7) * 16);
+            if (rmw) {
+              o[i].x += old[i].x; o[i].y += old[i].y; o[i].z += old[i].z; o[i].w += old[i].w;
             }
+          }
+          if (rmw && c + 1 < BN / 32) fetch_c(c + 1);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int rl = i * 4 + (lane >> 3);
+            if (row0 + rl >= p.M || ncol >= p.N) continue;
+            float* dst = gbase + static_cast<long long>(rl) * p.ldc + ncol;
+            if (p.split_k > 1)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(o[i].x),
+                           "f"(o[i].y), "f"(o[i].z), "f"(o[i].w)
+                           : "memory");
+            else
+              *reinterpret_cast<float4*>(dst) = o[i];
           }
           __syncwarp();
         }
@@ -998,7 +1088,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty_bar[acc]), 0));
+        else mbar_arrive(&tempty_bar[acc]);
+      }
       if (p.rs_on) {
         // the warp barrier orders every lane's stores before lane 0's system-scope release
         __syncwarp();
@@ -1012,9 +1105,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();  // nothing of the peer reads this CTA's shared memory or TMEM any more
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
@@ -1099,18 +1194,80 @@ static int make_tmap_mn4(CUtensorMap* tm, const void* ptr, uint64_t inner, uint6
 static int g_num_sms = 0;
 static int g_deterministic = 0;  // 1: no split-K (its atomics make the fp32 sum order vary)
 
-template <int A_MN, int B_MN, int FP8 = 0>
-static cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
-                          int grid, cudaStream_t stream) {
+template <int A_MN, int B_MN, int FP8, int TN, int PAIR = 0>
+static cudaError_t launch_tn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p,
+                             int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<A_MN, B_MN, FP8>,
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<A_MN, B_MN, FP8, TN, PAIR>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  gemm_bf16_tcgen05_kernel<A_MN, B_MN, FP8><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, p);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = GEMM_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = PAIR ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<A_MN, B_MN, FP8, TN, PAIR>, ta, tb, p);
+}
+template <int A_MN, int B_MN, int FP8 = 0>
+static cudaError_t launch(int tn, bool pair, const CUtensorMap& ta, const CUtensorMap& tb,
+                          const GemmParams& p, int grid, cudaStream_t stream) {
+  if (pair) return launch_tn<A_MN, B_MN, FP8, 256, 1>(ta, tb, p, grid, stream);
+  return tn == 128 ? launch_tn<A_MN, B_MN, FP8, 128>(ta, tb, p, grid, stream)
+                   : launch_tn<A_MN, B_MN, FP8, 256>(ta, tb, p, grid, stream);
+}
+
+// Tile shape and K-slices of a plain product, in units of one k-block of a 128 x 256 tile
+// (0.40 us).  Measured per k-block: 1.0 for that tile, 0.9 for a 256 x 256 tile on a CTA pair,
+// 0.75 for a 128 x 128 tile (its MMA reads as many operand bytes per cycle as shared memory
+// gives; it wins where it fills SMs the wide ones leave idle).  Units run in waves of `cap` CTAs
+// or cap / 2 pairs.  32768 x 6208 x 2048: 570 us single, 535 us on pairs, 804 us 128-wide;
+// 576 x 2048 x 5632: 44 / 38 / 36 us.
+// An fp32 accumulation may be cut in K, its slices meeting through vector reductions.  That pays
+// where one wave leaves SMs idle or all CTAs walk K in lockstep (a lone full wave runs its
+// k-blocks about 1.3 times slower: 2048 x 2048 x 32768 292 us whole, 210 us in two slices;
+// 1024 x 1024 x 16384 110 us whole, 41 us in four); with many waves it loses (32000 x 2048 x
+// 16384: 1.49 ms whole, 1.64 ms in two, 2.4 ms in eight), since a unit cannot be shorter than
+// its epilogue (about 30 blocks).
+struct TilePick {
+  int tn = 256, split = 1;
+  bool pair = false;
+};
+static TilePick pick_tiles(int M, int N, int num_kb, int batch, int cap, bool may_split) {
+  TilePick best;
+  double best_t = 1e30;
+  for (int kind = 0; kind < 3; ++kind) {  // 0: 128 x 256, 1: pair, 2: 128 x 128
+    const int tm = kind == 1 ? 2 * BM : BM, tn = kind == 2 ? 128 : 256;
+    const int slots = kind == 1 ? cap / 2 : cap;
+    const double c = kind == 0 ? 1.0 : kind == 1 ? 0.9 : 0.75;
+    if (slots < 1 || (kind == 1 && M <= BM)) continue;
+    const long long tiles = static_cast<long long>((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch;
+    for (int s = 1; s <= (may_split ? 8 : 1) && (s == 1 || s * 8 <= num_kb); ++s) {
+      const int kb = (num_kb + s - 1) / s;
+      if (s > 1 && static_cast<long long>(kb) * (s - 1) >= num_kb) continue;  // an empty slice
+      const long long waves = (tiles * s + slots - 1) / slots;
+      double unit = c * kb;
+      if (may_split && waves == 1 && tiles * s * 2 > slots) unit *= 1.3;
+      if (s > 1 && waves > 1 && unit < 30.0) unit = 30.0;
+      const double t = s > 1 ? 1.07 * waves * unit + 30.0 : waves * unit + 8.0;
+      if (t < best_t * 0.98) {  // a near tie keeps the earlier kind and fewer slices
+        best_t = t;
+        best.tn = tn;
+        best.split = s;
+        best.pair = kind == 1;
+      }
+    }
+  }
+  return best;
 }
 
 }  // namespace ceo
@@ -1123,7 +1280,7 @@ struct Fp8Desc {
   const float* scale_b = nullptr;
 };
 
-// SwiGLU fused into the epilogue (see GemmParams::epi_mode).
+// SwiGLU fused into the epilogue (see GemmParams::epi_mode), and the residual's factor.
 struct EpiDesc {
   int mode = 0;
   void* aux = nullptr;
@@ -1171,6 +1328,18 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
+  int cap = g_num_sms;
+  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
+  TilePick pick;
+  if (fz.kind == 0) {
+    const int bke = f8.on ? 2 * BK : BK;
+    pick = pick_tiles(M, N, (K + bke - 1) / bke, batch, cap,
+                      out_f32 && accumulate && !bias && !residual && split_k_mode != 0 &&
+                          !ceo::g_deterministic);
+  }
+  const int BN = pick.tn, split = pick.split;  // this call's tile width and K-slices
+  const bool pair = pick.pair;                 // a CTA pair per 256 x 256 tile
+  const int BROWS = pair ? BN / 2 : BN, TM = pair ? 2 * BM : BM;
   CUtensorMap ta, tb;
   int rc;
   const bool a4 = a_mn_major && fz.kind == 0 && (M & 63) == 0;
@@ -1183,9 +1352,9 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
     rc = make_tmap(&ta, A, M, K, batch, lda, batch_stride_a, BK);
   if (rc) return -3;
   if (b_mn_major == 0)
-    rc = make_tmap(&tb, B, K, N, batch, ldb, batch_stride_b, BN, esize);
+    rc = make_tmap(&tb, B, K, N, batch, ldb, batch_stride_b, BROWS, esize);
   else if (b4)
-    rc = make_tmap_mn4(&tb, B, N, K, batch, ldb, batch_stride_b, BN / 64);
+    rc = make_tmap_mn4(&tb, B, N, K, batch, ldb, batch_stride_b, BROWS / 64);
   else
     rc = make_tmap(&tb, B, N, K, batch, ldb, batch_stride_b, BK);
   if (rc) return -4;
@@ -1210,7 +1379,7 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   p.fp8_b = f8.kind_b;
   p.scale_a = f8.scale_a;
   p.scale_b = f8.scale_b;
-  p.num_m = (M + BM - 1) / BM;
+  p.num_m = (M + TM - 1) / TM;
   p.num_n = (N + BN - 1) / BN;
   p.status = status;
   p.rank = fz.rank;
@@ -1244,9 +1413,8 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   }
   // bands of 16 row blocks: a wave of 148 tiles is then ~16 x 9 tiles whose A and B panels
   // both stay in L2 (m-fastest over all rows re-reads A once per ~2 n-blocks)
-  p.grp_m = p.num_m > 16 ? 16 : p.num_m;
-  int cap = g_num_sms;
-  if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
+  const int band = 16 * BM / TM;
+  p.grp_m = p.num_m > band ? band : p.num_m;
   if (fz.kind == 1 || fz.kind == 2) {
     // gathered operand: K-major rows only, shards of whole row blocks, dense rows
     const int rows = fz.kind == 1 ? M : N;
@@ -1313,30 +1481,16 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
     p.grp_m = p.num_m;
   }
   long long total = static_cast<long long>(p.num_m) * p.num_n * batch;
-  p.split_k = 1;
-  if (fz.kind == 0 && out_f32 && accumulate && !bias && !residual && split_k_mode != 0 &&
-      !ceo::g_deterministic) {
-    // few tiles with a long K (weight gradients): pick the split that fills whole waves best
-    const int bke = f8.on ? 2 * BK : BK;
-    const int num_kb = (K + bke - 1) / bke;
-    // every extra slice re-sends the whole fp32 C through L2 atomics, so a split has to buy a
-    // clear gain in wave efficiency (measured: 5 slices of the 2048x5632 gradient lose)
-    double best = 0.0;
-    for (int s = 1; s <= 3 && s * 16 <= num_kb; ++s) {
-      const long long units = total * s;
-      const long long waves = (units + cap - 1) / cap;
-      const double eff = static_cast<double>(units) / (waves * cap) - 0.05 * (s - 1);
-      if (eff > best + (s > 1 ? 0.05 : 0.0)) { best = eff; p.split_k = s; }
-    }
-  }
+  p.split_k = split;
   total *= p.split_k;
   int grid = static_cast<int>(total + p.ag_ctas < cap ? total + p.ag_ctas : cap);
+  if (pair) grid = 2 * static_cast<int>(total < cap / 2 ? total : cap / 2);
   cudaError_t e;
-  if (f8.on) e = launch<0, 0, 1>(ta, tb, p, grid, stream);
-  else if (a_mn_major == 0 && b_mn_major == 0) e = launch<0, 0>(ta, tb, p, grid, stream);
-  else if (a_mn_major == 0) e = launch<0, 1>(ta, tb, p, grid, stream);
-  else if (b_mn_major == 0) e = launch<1, 0>(ta, tb, p, grid, stream);
-  else e = launch<1, 1>(ta, tb, p, grid, stream);
+  if (f8.on) e = launch<0, 0, 1>(BN, pair, ta, tb, p, grid, stream);
+  else if (a_mn_major == 0 && b_mn_major == 0) e = launch<0, 0>(BN, pair, ta, tb, p, grid, stream);
+  else if (a_mn_major == 0) e = launch<0, 1>(BN, pair, ta, tb, p, grid, stream);
+  else if (b_mn_major == 0) e = launch<1, 0>(BN, pair, ta, tb, p, grid, stream);
+  else e = launch<1, 1>(BN, pair, ta, tb, p, grid, stream);
   return static_cast<int>(e);
 }
 
