@@ -47,7 +47,8 @@ def _form(model):
     dev = model.embed_tokens.device
     if (dev.type != "cuda" or torch.cuda.current_device() != dev.index
             or not matmul_ops.FUSED_SWIGLU or c.activation != "swiglu"
-            or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks):
+            or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks
+            or torch.autograd.forward_ad._current_level >= 0):  # tangents: refused further down
         return None
     D, V, F = c.hidden_dim, c.vocab_size, c.intermediate_dim
     H, d = c.num_heads, c.head_dim
