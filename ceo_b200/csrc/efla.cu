@@ -54,6 +54,48 @@ __device__ __forceinline__ void frag_store_bf16(bf16* base, long long ld, float 
   }
 }
 
+// The same rows as 16-byte stores (base 16-byte aligned, ld a multiple of 8): the four lanes of a
+// row exchange their pairs, a 4 x 4 transpose in two shuffle rounds, so that a lane holds eight
+// neighbouring columns.  A 4-byte store touches eight rows for 16 bytes each, and these kernels
+// are bound by the L1 pipe (85 % busy): a quarter of the store instructions, whole sectors.
+template <int NT>
+__device__ __forceinline__ void frag_store_bf16x8(bf16* base, long long ld, float (*acc)[4]) {
+  static_assert(NT % 4 == 0, "groups of 32 columns");
+  const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
+  const bool b0 = tg & 1, b1 = tg & 2;
+#pragma unroll
+  for (int q = 0; q < NT / 4; ++q)
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      uint32_t r[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bf162 v = __floats2bfloat162_rn(acc[4 * q + j][2 * hf], acc[4 * q + j][2 * hf + 1]);
+        r[j] = *reinterpret_cast<const uint32_t*>(&v);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        const uint32_t x = __shfl_xor_sync(0xffffffffu, b0 ? r[j] : r[j + 1], 1);
+        if (b0) r[j] = x;
+        else r[j + 1] = x;
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint32_t x = __shfl_xor_sync(0xffffffffu, b1 ? r[j] : r[j + 2], 2);
+        if (b1) r[j] = x;
+        else r[j + 2] = x;
+      }
+      *reinterpret_cast<uint4*>(base + (g + 8 * hf) * ld + (4 * q + tg) * 8) =
+          make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+// Rows of a caller's tensor: wide stores where its alignment allows them.
+template <int NT>
+__device__ __forceinline__ void frag_store_any(bf16* base, long long ld, float (*acc)[4]) {
+  if (((reinterpret_cast<uintptr_t>(base) | (ld * 2)) & 15) == 0) frag_store_bf16x8<NT>(base, ld, acc);
+  else frag_store_bf16<NT>(base, ld, acc);
+}
+
 // ---- tiles moved by TMA ------------------------------------------------------------------
 // Token-major tensors (q, k, v, w, u, ...) are mapped as matrices [B*T][H*D] with the token
 // stride as leading dimension, the state snapshots as [B*H*n*D][D]; both with 64-column boxes
@@ -120,25 +162,42 @@ __device__ __forceinline__ void wg(float (*acc)[4], const SwzTile& A, int m0, co
 //
 // C[i][j0..j0+3] = sign * rs[i] * sum_kk A[i][kk] * B[kk][j0..], for `nblk` independent N x N
 // blocks whose operands sit `step` elements apart.
+// A thread owns R rows x 4 columns and reads A four kk at a time: the products are bound by
+// shared-memory reads, and R = 2 shares every read of B (at N = 16 there are only enough outputs
+// for one row per thread).
 template <int NTHR, int N>
 __device__ __forceinline__ void solve_block_prod(const float* A, const float* B, float* C,
                                                  const float* rs, float sign, int nblk,
                                                  int step) {
-  constexpr int Q = N / 4;
-  for (int o = threadIdx.x; o < nblk * N * Q; o += NTHR) {
-    const int blk = o / (N * Q), rem = o - blk * N * Q, i = rem / Q, j0 = (rem - i * Q) * 4;
+  constexpr int R = N >= 32 ? 2 : 1, Q = N / 4, PER = N / R * Q;
+  for (int o = threadIdx.x; o < nblk * PER; o += NTHR) {
+    const int blk = o / PER, rem = o - blk * PER, i = rem / Q * R, j0 = (rem % Q) * 4;
     const float* a = A + blk * step + i * GLD;
     const float* bb = B + blk * step + j0;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 acc[R];
 #pragma unroll
-    for (int kk = 0; kk < N; ++kk) {
-      const float av = a[kk];
-      const float4 bv = *reinterpret_cast<const float4*>(bb + kk * GLD);
-      acc.x += av * bv.x; acc.y += av * bv.y; acc.z += av * bv.z; acc.w += av * bv.w;
+    for (int r = 0; r < R; ++r) acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k4 = 0; k4 < N; k4 += 4) {
+      float4 av[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) av[r] = *reinterpret_cast<const float4*>(a + r * GLD + k4);
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        const float4 bv = *reinterpret_cast<const float4*>(bb + (k4 + kk) * GLD);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const float x = kk == 0 ? av[r].x : kk == 1 ? av[r].y : kk == 2 ? av[r].z : av[r].w;
+          acc[r].x += x * bv.x; acc[r].y += x * bv.y; acc[r].z += x * bv.z; acc[r].w += x * bv.w;
+        }
+      }
     }
-    const float f = rs ? sign * rs[blk * (step / (GLD + 1)) + i] : sign;
-    *reinterpret_cast<float4*>(C + blk * step + i * GLD + j0) =
-        make_float4(f * acc.x, f * acc.y, f * acc.z, f * acc.w);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float f = rs ? sign * rs[blk * (step / (GLD + 1)) + i + r] : sign;
+      *reinterpret_cast<float4*>(C + blk * step + (i + r) * GLD + j0) =
+          make_float4(f * acc[r].x, f * acc[r].y, f * acc[r].z, f * acc[r].w);
+    }
   }
 }
 
@@ -246,9 +305,10 @@ efla_wy_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int row = 16 * warp + g + (e >> 1) * 8, col = nt * 8 + 2 * tg + (e & 1);
-        Gs[row * GLD + col] = col < row ? acc[nt][e] : 0.f;
+      for (int hf = 0; hf < 2; ++hf) {
+        const int row = 16 * warp + g + hf * 8, col = nt * 8 + 2 * tg;
+        *reinterpret_cast<float2*>(Gs + row * GLD + col) =
+            make_float2(col < row ? acc[nt][2 * hf] : 0.f, col + 1 < row ? acc[nt][2 * hf + 1] : 0.f);
       }
   }
   if (threadIdx.x < CH) al[threadIdx.x] = my_al;
@@ -276,14 +336,14 @@ efla_wy_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__
     float acc[D / 8][4];
     zero_acc<D / 8>(acc);
     wg<D / 8, CH, false, true>(acc, Tt, 16 * warp, Kt, 0);
-    frag_store_bf16<D / 8>(w + orow * D, static_cast<long long>(H) * D, acc);
+    frag_store_any<D / 8>(w + orow * D, static_cast<long long>(H) * D, acc);
   }
   tile_wait(&bars[1], status);
   {
     float acc[D / 8][4];
     zero_acc<D / 8>(acc);
     wg<D / 8, CH, false, true>(acc, Tt, 16 * warp, Vt, 0);
-    frag_store_bf16<D / 8>(u + orow * D, static_cast<long long>(H) * D, acc);
+    frag_store_any<D / 8>(u + orow * D, static_cast<long long>(H) * D, acc);
   }
 }
 
@@ -595,7 +655,7 @@ efla_out_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   zero_acc<NT>(acc);
   wg<NT, D, false, true>(acc, Qt, 16 * r, St, c0);
   wg<NT, CH, false, true>(acc, Pt, 16 * r, Upt, c0);
-  frag_store_bf16<NT>(o + (static_cast<long long>(tok0) + 16 * r) * HD + h * D + c0, HD, acc);
+  frag_store_any<NT>(o + (static_cast<long long>(tok0) + 16 * r) * HD + h * D + c0, HD, acc);
 }
 
 // ===================================================== forward: O on tcgen05 (D = 128)
@@ -866,13 +926,13 @@ efla_bwd_local_kernel(const __grid_constant__ CUtensorMap tm_q,
     zero_acc<NT>(acc);
     wg<NT, D, false, false>(acc, dOt, 16 * r, St, c0);
     wg<NT, CH, false, true>(acc, dPt, 16 * r, Kt, c0);
-    frag_store_bf16<NT>(dq + (static_cast<long long>(tok0) + 16 * r) * dqs + h * D + c0, dqs, acc);
+    frag_store_any<NT>(dq + (static_cast<long long>(tok0) + 16 * r) * dqs + h * D + c0, dqs, acc);
   }
   {
     float acc[NT][4];
     zero_acc<NT>(acc);
     wg<NT, CH, true, true>(acc, Pt, 16 * r, dOt, c0);
-    frag_store_bf16<NT>(dloc + (static_cast<long long>(tok0) + 16 * r) * HD + h * D + c0, HD, acc);
+    frag_store_any<NT>(dloc + (static_cast<long long>(tok0) + 16 * r) * HD + h * D + c0, HD, acc);
   }
 }
 
@@ -1248,7 +1308,7 @@ efla_bwd_final_kernel(const __grid_constant__ CUtensorMap tm_q,
   wg<NT, CH, true, true>(kacc, dPt, 16 * r, Qt, c0);
   tile_wait(&bars[4], status);
   wg<NT, D, false, false>(kacc, Upt, 16 * r, dSt, c0);
-  frag_store_bf16<NT>(dk + (static_cast<long long>(tok0) + 16 * r) * dks + h * D + c0, dks, kacc);
+  frag_store_any<NT>(dk + (static_cast<long long>(tok0) + 16 * r) * dks + h * D + c0, dks, kacc);
   if (threadIdx.x < CH)
     dalpha[(static_cast<long long>(tok0) + threadIdx.x) * H + h] = dal[threadIdx.x];
 }
