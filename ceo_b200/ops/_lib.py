@@ -129,7 +129,8 @@ def check(rc: int, what: str) -> None:
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle, without building a Stream object (two microseconds a launch)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: torch.Tensor | None) -> int | None:
