@@ -1,6 +1,8 @@
 // See skinny.cuh for the design.  Warp 0 is the TMA producer, warp 1 issues the MMAs, warps
 // 2..5 (one TMEM lane quadrant each) move the accumulator to shared memory, where the cluster's
 // partial sums are added and written out.
+#include <atomic>
+
 #include "common/ptx.cuh"
 #include "common/tmap.h"
 #include "common/util.cuh"
@@ -213,9 +215,17 @@ static cudaError_t skinny_launch(const CUtensorMap& tw, const CUtensorMap& ta,
                                  const SkinnyKernelArgs& p, int S, int tiles, cudaStream_t stream) {
   constexpr int SMEM = STG * (SK_W_BYTES + NB * SK_BK * 2) + 1024 + 256;
   static_assert(STG * (SK_W_BYTES + NB * SK_BK * 2) >= NB * SK_ROWS * 4, "partial sums fit the ring");
-  const cudaError_t e0 = cudaFuncSetAttribute(skinny_gemm_kernel<NB, STG>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  int dev = 0;
+  cudaError_t e0 = cudaGetDevice(&dev);
   if (e0 != cudaSuccess) return e0;
+  static std::atomic<unsigned long long> configured{0};  // one bit per device
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev >= 64 || !(configured.load(std::memory_order_relaxed) & bit)) {
+    e0 = cudaFuncSetAttribute(skinny_gemm_kernel<NB, STG>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e0 != cudaSuccess) return e0;
+    configured.fetch_or(bit, std::memory_order_relaxed);
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S, tiles, 1);
   cfg.blockDim = dim3(SK_THREADS, 1, 1);
