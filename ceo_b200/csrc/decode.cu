@@ -8,6 +8,9 @@
 // way.  Only activations wait for the previous kernel.  The chain is safe because the first
 // kernel (the embedding gather) is an ordinary launch: everything the stream held before is
 // complete, and no kernel of the chain writes a weight.
+//
+// Per step, layers from Python -> this loop: 1.3B, one sequence, 11.7 -> 0.96 ms; 340M, 40
+// sequences, 11.8 -> 0.92 ms; 7B, 7 sequences, 15.9 -> 3.46 ms (4.1 TB/s).
 #include "common/ptx.cuh"
 #include "common/util.cuh"
 #include "include/ceo_kernels.h"
