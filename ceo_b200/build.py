@@ -29,11 +29,16 @@ LIB_CHK = ROOT / "lib" / "libceo_b200_chk.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-lineinfo", "-O3", "-std=c++17", "--use_fast_math",
+    "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=default",
     "--expt-relaxed-constexpr",
     f"-I{CSRC}",
 ]
+FAST_MATH = ["--use_fast_math"]
+# units that need an accurate exponential (csrc/common/sigmoid.cuh): what --use_fast_math implies,
+# without its replacement of the math functions
+ACCURATE = {"efla_prep"}
+ACCURATE_MATH = ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"]
 
 
 def _nvcc() -> str:
@@ -57,7 +62,8 @@ def _compile(src: Path, hdr_mtime: float, verbose: bool, extra: list[str],
     obj = objdir / (src.stem + ".o")
     if obj.exists() and obj.stat().st_mtime > max(src.stat().st_mtime, hdr_mtime) and not extra:
         return obj, ""
-    cmd = [_nvcc(), *NVCC_FLAGS, *extra, "-c", str(src), "-o", str(obj)]
+    math = ACCURATE_MATH if src.stem in ACCURATE else FAST_MATH
+    cmd = [_nvcc(), *NVCC_FLAGS, *math, *extra, "-c", str(src), "-o", str(obj)]
     if verbose:
         cmd.insert(1, "-Xptxas")
         cmd.insert(2, "-v")

@@ -121,6 +121,46 @@ def test_beta_logits_in_prep(H, d, P, pad, rows):
     assert dl[:, :P * H * d].isnan().all()
 
 
+@pytest.mark.parametrize("d,normalize", [(64, 1), (128, 0)])
+def test_beta_and_its_gradient_are_those_of_torch_sigmoid(d, normalize):
+    # every finite bf16 logit whose exponential is a normal fp32 number, bit for bit: a last bit
+    # of beta decides roundings in all layers behind it
+    x = torch.arange(-2 ** 15, 2 ** 15, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = x[x.isfinite() & (x.float().abs() < 87)].cuda()
+    H = 8
+    x = x[:x.numel() // H * H].view(-1, H)
+    rows = x.shape[0]
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q = torch.randn(rows, H, d, device="cuda", generator=g).bfloat16()
+    dqn, dkn = (torch.randn(rows, H, d, device="cuda", generator=g).bfloat16() for _ in range(2))
+    da = torch.randn(rows, H, device="cuda", generator=g)
+    beta = torch.sigmoid(x.float())
+    L, st = _lib.lib(), _lib.stream()
+    new = lambda *s, dt=torch.float32: torch.empty(*s, dtype=dt, device="cuda")
+    half = lambda: new(rows, H, d, dt=torch.bfloat16)
+    qn, kn, rq, rk, al, al2, bo = half(), half(), *(new(rows, H) for _ in range(5))
+    _lib.check(L.ceo_efla_prep_fwd_logits(
+        q.data_ptr(), q.data_ptr(), x.data_ptr(), H, bo.data_ptr(), qn.data_ptr(), kn.data_ptr(),
+        rq.data_ptr(), rk.data_ptr(), al.data_ptr(), rows, H, d, H * d, H * d, normalize, st), "prep")
+    assert torch.equal(bo, beta)
+    _lib.check(L.ceo_efla_prep_fwd(
+        q.data_ptr(), q.data_ptr(), beta.data_ptr(), 0, qn.data_ptr(), kn.data_ptr(), rq.data_ptr(),
+        rk.data_ptr(), al2.data_ptr(), rows, H, d, H * d, H * d, normalize, st), "prep")
+    assert torch.equal(al, al2)
+    dq, dk, db, dl = half(), half(), new(rows, H), torch.empty_like(x)
+    _lib.check(L.ceo_efla_prep_bwd_logits(
+        dqn.data_ptr(), dkn.data_ptr(), qn.data_ptr(), kn.data_ptr(), rq.data_ptr(), rk.data_ptr(),
+        beta.data_ptr(), da.data_ptr(), dq.data_ptr(), dk.data_ptr(), dl.data_ptr(), H, 0, rows, H, d,
+        H * d, H * d, normalize, st), "prep_bwd")
+    _lib.check(L.ceo_efla_prep_bwd(
+        dqn.data_ptr(), dkn.data_ptr(), qn.data_ptr(), kn.data_ptr(), rq.data_ptr(), rk.data_ptr(),
+        beta.data_ptr(), 0, da.data_ptr(), dq.data_ptr(), dk.data_ptr(), db.data_ptr(), rows, H, d,
+        H * d, H * d, normalize, st), "prep_bwd")
+    want = db * beta * (1.0 - beta)
+    sure = want.abs() > 1e-30  # (the kernels flush denormals)
+    assert torch.equal(dl[sure], want.bfloat16()[sure]) and not dl[~sure].float().abs().gt(2e-30).any()
+
+
 @pytest.mark.parametrize("D", [512, 1024, 2048, 4096, 768])
 @pytest.mark.parametrize("rows", [1, 3, 4, 5, 2500])
 def test_rmsnorm_rows(D, rows):
