@@ -546,12 +546,14 @@ efla_state_fwd_kernel(const __grid_constant__ CUtensorMap tm_k,
 }
 
 // Incoming state of every span from the spans' maps: s[0] = s0, s[1] = R[0] (span 0 ran from
-// s0), s[j + 1] = P[j] s[j] + R[j].  One CTA per (sequence, head, 8 value columns), the state
+// s0), s[j + 1] = P[j] s[j] + R[j], and R[j] alone where a document starts inside span j: P[j] is
+// zero there, but zero times a state that overflowed in an earlier document is NaN.  One CTA per (sequence, head, 8 value columns), the state
 // slice in shared memory; thread (row, half) adds half of the 8 columns of one row in fp32.
 template <int D>
 __global__ void __launch_bounds__(2 * D)
 efla_fold_kernel(const float* __restrict__ s0, const float* __restrict__ P,
-                 const float* __restrict__ R, float* __restrict__ s_in, int segs) {
+                 const float* __restrict__ R, const unsigned char* __restrict__ resets,
+                 float* __restrict__ s_in, int segs, int n, int H) {
   __shared__ float4 ss[D][2];
   const long long bh = blockIdx.y;
   const int row = threadIdx.x >> 1, half = threadIdx.x & 1, col = blockIdx.x * 8 + half * 4;
@@ -571,18 +573,23 @@ efla_fold_kernel(const float* __restrict__ s0, const float* __restrict__ P,
         asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                      : "=f"(pr[k].x), "=f"(pr[k].y), "=f"(pr[k].z), "=f"(pr[k].w)
                      : "l"(prow + k));
-      __syncthreads();  // the previous step's reads are over
-      ss[row][half] = s;
-      __syncthreads();
+      int cut = 0;  // a document starts in this span
+      if (resets)
+        for (int c = j * n / segs + threadIdx.x; c < (j + 1) * n / segs; c += 2 * D)
+          cut |= resets[bh / H * n + c];
+      if (!__syncthreads_or(cut)) {  // (also: the previous step's reads are over)
+        ss[row][half] = s;
+        __syncthreads();
 #pragma unroll
-      for (int k = 0; k < D / 4; ++k) {
-        const float4 pv = pr[k];
-        const float4 a = ss[4 * k][half], b = ss[4 * k + 1][half], c = ss[4 * k + 2][half],
-                     d = ss[4 * k + 3][half];
-        acc.x += pv.x * a.x + pv.y * b.x + pv.z * c.x + pv.w * d.x;
-        acc.y += pv.x * a.y + pv.y * b.y + pv.z * c.y + pv.w * d.y;
-        acc.z += pv.x * a.z + pv.y * b.z + pv.z * c.z + pv.w * d.z;
-        acc.w += pv.x * a.w + pv.y * b.w + pv.z * c.w + pv.w * d.w;
+        for (int k = 0; k < D / 4; ++k) {
+          const float4 pv = pr[k];
+          const float4 a = ss[4 * k][half], b = ss[4 * k + 1][half], c = ss[4 * k + 2][half],
+                       d = ss[4 * k + 3][half];
+          acc.x += pv.x * a.x + pv.y * b.x + pv.z * c.x + pv.w * d.x;
+          acc.y += pv.x * a.y + pv.y * b.y + pv.z * c.y + pv.w * d.y;
+          acc.z += pv.x * a.z + pv.y * b.z + pv.z * c.z + pv.w * d.z;
+          acc.w += pv.x * a.w + pv.y * b.w + pv.z * c.w + pv.w * d.w;
+        }
       }
     }
     s = acc;
@@ -1399,7 +1406,8 @@ static int efla_state_segmented(const CUtensorMap* m, const EflaTensors& t, int 
   float *R = t.seg_ws, *P = R + one, *s_in = P + one;
   const float* s0 = static_cast<const float*>(t.p[I_S0]);
   efla_state_launch<D>(m, dim3(2 * (D / BV), B * H * G), s0, R, P, t, T, H, G, 1, st);
-  efla_fold_kernel<D><<<dim3(D / 8, B * H), 2 * D, 0, st>>>(s0, P, R, s_in, G);
+  efla_fold_kernel<D><<<dim3(D / 8, B * H), 2 * D, 0, st>>>(
+      s0, P, R, static_cast<const unsigned char*>(t.p[I_RESETS]), s_in, G, T / CH, H);
   efla_state_launch<D>(m, dim3(D / BV, B * H * G), s_in,
                        static_cast<float*>(const_cast<void*>(t.p[I_SFINAL])), nullptr, t, T, H, G,
                        0, st);
