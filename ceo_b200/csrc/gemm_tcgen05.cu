@@ -352,6 +352,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
   }
   tc_fence_before();
   __syncthreads();
+  __syncwarp();  // (the cluster barrier and the TMEM instructions are warp-aligned)
   if (PAIR) cluster_sync();  // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
@@ -1105,6 +1106,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA,
 
   tc_fence_before();
   __syncthreads();
+  __syncwarp();
   if (PAIR) cluster_sync();  // nothing of the peer reads this CTA's shared memory or TMEM any more
   if (warp == 1) {
     tc_fence_after();

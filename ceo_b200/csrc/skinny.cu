@@ -202,6 +202,9 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
   }
+  // the loop above leaves its lanes at different times, and both the cluster barrier and the
+  // TMEM release below are warp-aligned instructions
+  __syncwarp();
   // no CTA leaves while another one may still read its partial sums
   if (S > 1) cluster_sync_all();
   if (warp == 1) {
