@@ -22,6 +22,22 @@ __device__ __forceinline__ void dec_pdl_wait() { asm volatile("griddepcontrol.wa
 __device__ __forceinline__ void dec_pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Activations of the chain: the kernel before may still be writing them when this one is already
+// resident, so they are no read-only data (`const __restrict__` or __ldg would say so, and such
+// loads may move across the wait).  These loads are neither moved nor non-coherent.
+__device__ __forceinline__ uint4 ld_act16(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_act(const bf16* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+  return __uint_as_float(static_cast<uint32_t>(v) << 16);
+}
 
 // ------------------------------------------------------------------- embedding
 __global__ void __launch_bounds__(128)
@@ -39,8 +55,7 @@ decode_embed_kernel(const long long* __restrict__ ids, const bf16* __restrict__ 
 constexpr int DN_THREADS = 256;
 constexpr int DN_MAXV = 4;  // 8-element vectors per thread: D <= 8192
 __global__ void __launch_bounds__(DN_THREADS)
-decode_rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                      bf16* __restrict__ y, int D, float eps) {
+decode_rmsnorm_kernel(const bf16* x, const bf16* __restrict__ w, bf16* y, int D, float eps) {
   __shared__ float red[33];
   const int nv = D >> 3;
   dec_pdl_trigger();
@@ -51,14 +66,20 @@ decode_rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
     if (c < nv) wp[i] = reinterpret_cast<const uint4*>(w)[c];
   }
   dec_pdl_wait();
-  const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<long long>(blockIdx.x) * D);
+  const bf16* xr = x + static_cast<long long>(blockIdx.x) * D;
+  uint4 xp[DN_MAXV];
+#pragma unroll
+  for (int i = 0; i < DN_MAXV; ++i) {
+    const int c = threadIdx.x + i * DN_THREADS;
+    if (c < nv) xp[i] = ld_act16(xr + c * 8);
+  }
   float v[DN_MAXV][8];
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < DN_MAXV; ++i) {
     const int c = threadIdx.x + i * DN_THREADS;
     if (c < nv) {
-      unpack8(xr[c], v[i]);
+      unpack8(xp[i], v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) ss += v[i][j] * v[i][j];
     }
@@ -90,9 +111,9 @@ decode_rmsnorm_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
 constexpr int DR_TOK = 16;
 template <int D>
 __global__ void __launch_bounds__(128)
-decode_delta_kernel(const bf16* __restrict__ proj, long long ldp, int P, int H,
-                    const float* __restrict__ beta_scalar, int normalize,
-                    float* __restrict__ state, bf16* __restrict__ o, int T) {
+decode_delta_kernel(const bf16* proj, long long ldp, int P, int H,
+                    const float* __restrict__ beta_scalar, int normalize, float* state, bf16* o,
+                    int T) {
   constexpr int RT = D / 4;  // state rows per thread
   __shared__ __align__(16) float ks[DR_TOK][D], qs[DR_TOK][D];
   __shared__ float vs[DR_TOK][32], al[DR_TOK], kq[DR_TOK];
@@ -127,14 +148,13 @@ decode_delta_kernel(const bf16* __restrict__ proj, long long ldp, int P, int H,
       float qv[E], kv[E], sq = 0.f, sk = 0.f;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        qv[e] = __bfloat162float(row[lane + 32 * e]);
-        kv[e] = P == 3 ? __bfloat162float(row[hd + lane + 32 * e]) : qv[e];
+        qv[e] = ld_act(row + lane + 32 * e);
+        kv[e] = P == 3 ? ld_act(row + hd + lane + 32 * e) : qv[e];
         sq += qv[e] * qv[e];
         sk += kv[e] * kv[e];
       }
-      if (lane < 32) vs[t][lane] = __bfloat162float(row[(P - 1) * hd + blockIdx.x * 32 + lane]);
-      const float bl = beta_scalar ? beta_scalar[0]
-                                   : __bfloat162float(row[P * hd - h * D + h]);
+      vs[t][lane] = ld_act(row + (P - 1) * hd + blockIdx.x * 32 + lane);
+      const float bl = beta_scalar ? beta_scalar[0] : ld_act(row + P * hd - h * D + h);
       sq = warp_reduce_sum(sq);
       sk = warp_reduce_sum(sk);
       const float iq = normalize ? rsqrtf(sq + 1e-6f) : 1.f;

@@ -21,3 +21,16 @@ def test_warps_are_whole_at_aligned_instructions(name, call):
     assert len(at) == 2
     for i in at:
         assert "__syncwarp();" in lines[i - 1], lines[i - 2:i + 1]
+
+
+# A programmatic dependent launch is resident while the kernel before it still writes its inputs:
+# of a chain kernel's pointers only weights may be declared read-only.
+@pytest.mark.parametrize("kernel,weights", [("decode_rmsnorm_kernel", {"w"}),
+                                            ("decode_delta_kernel", {"beta_scalar"})])
+def test_chain_kernels_promise_read_only_weights_alone(kernel, weights):
+    text = _code("decode.cu")
+    params = re.search(kernel + r"\(([^)]*)\)\s*\{", text).group(1)
+    fixed = {p.split()[-1] for p in params.split(",") if "const" in p and "__restrict__" in p}
+    assert fixed == weights
+    body = text[text.index(params):].split("\n}\n")[0]
+    assert "__ldg" not in body and "ld.global.nc" not in body
