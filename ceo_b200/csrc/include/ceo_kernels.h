@@ -403,6 +403,7 @@ int ceo_zero_bucket_reduce(void* const* grads, void* const* flags, const void* r
 int ceo_set_wait_limit(unsigned int iterations);
 int ceo_gemm_set_wait_limit(unsigned int iterations);
 int ceo_efla_set_wait_limit(unsigned int iterations);
+int ceo_skinny_set_wait_limit(unsigned int iterations);
 
 #ifdef __cplusplus
 }

@@ -6,6 +6,7 @@
 #include "common/ptx.cuh"
 #include "common/tmap.h"
 #include "common/util.cuh"
+#include "include/ceo_kernels.h"
 #include "skinny.cuh"
 
 namespace ceo {
@@ -295,3 +296,8 @@ int skinny_gemm(const SkinnyArgs& a, cudaStream_t stream) {
 }
 
 }  // namespace ceo
+
+// See ceo_set_wait_limit.
+extern "C" int ceo_skinny_set_wait_limit(unsigned int iterations) {
+  return ceo::set_wait_limit_override(iterations);
+}

@@ -4,6 +4,8 @@ from pathlib import Path
 
 import pytest
 
+from ceo_b200.runtime.fault import describe_status
+
 CSRC = Path(__file__).resolve().parent.parent / "ceo_b200" / "csrc"
 
 
@@ -34,3 +36,18 @@ def test_chain_kernels_promise_read_only_weights_alone(kernel, weights):
     assert fixed == weights
     body = text[text.index(params):].split("\n}\n")[0]
     assert "__ldg" not in body and "ld.global.nc" not in body
+
+
+# The limit of bounded waits is kept per translation unit: ceo_set_wait_limit has to reach each
+# unit that waits, and each code such a unit writes needs a name.
+def test_wait_limit_and_status_codes_reach_every_unit():
+    forward = re.search(r"int ceo_set_wait_limit\(unsigned int iterations\) \{(.*?)\n\}",
+                        _code("comm.cu"), re.S).group(1)
+    for src in sorted(CSRC.glob("*.cu")):
+        text = _code(src.name)
+        if not re.search(r"\b(mbar_wait|wait_limit)\(", text):
+            continue
+        own = re.findall(r"(\w+)\(unsigned int iterations\) \{\s*return ceo::set_wait_limit", text)
+        assert src.name == "comm.cu" or (len(own) == 1 and own[0] + "(iterations)" in forward), src
+        for code in re.findall(r"\b\w*STATUS = (0x[0-9A-Fa-f]+);", text):
+            assert "status" not in describe_status(int(code, 16)), (src, code)
