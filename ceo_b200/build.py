@@ -37,7 +37,7 @@ NVCC_FLAGS = [
 FAST_MATH = ["--use_fast_math"]
 # units that need an accurate exponential (csrc/common/sigmoid.cuh): what --use_fast_math implies,
 # without its replacement of the math functions
-ACCURATE = {"efla_prep"}
+ACCURATE = {"decode", "efla_prep"}
 ACCURATE_MATH = ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"]
 
 

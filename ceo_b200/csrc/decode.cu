@@ -12,6 +12,7 @@
 // Per step, layers from Python -> this loop: 1.3B, one sequence, 11.7 -> 0.96 ms; 340M, 40
 // sequences, 11.8 -> 0.92 ms; 7B, 7 sequences, 15.9 -> 3.46 ms (4.1 TB/s).
 #include "common/ptx.cuh"
+#include "common/sigmoid.cuh"
 #include "common/util.cuh"
 #include "include/ceo_kernels.h"
 #include "skinny.cuh"
@@ -170,7 +171,7 @@ decode_delta_kernel(const bf16* proj, long long ldp, int P, int H,
       }
       dot = warp_reduce_sum(dot);
       if (lane == 0) {
-        const float beta = beta_scalar ? bl : 1.f / (1.f + __expf(-bl));
+        const float beta = beta_scalar ? bl : sigmoid_f32(bl);
         al[t] = normalize ? -expm1f(-beta) : efla_coeff(beta, sk);
         kq[t] = dot;
       }

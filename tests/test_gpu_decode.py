@@ -92,6 +92,31 @@ def test_native_decode_matches_layers(d, per_token, use_query, normalize, monkey
         assert (a - b).norm() / b.norm() < 2e-2
 
 
+def test_decode_beta_is_torch_sigmoid():
+    # one head whose key and value are the first unit vector and ones, so that row 0 of the state
+    # after one token is alpha itself, bit for bit; 128 tokens spell 128 logits in binary
+    cfg = Config.parse_from_file("configs/efla_340m.yaml").model
+    cfg.num_layers, cfg.vocab_size, cfg.hidden_dim, cfg.intermediate_dim = 1, 128, 64, 32
+    cfg.num_heads, cfg.head_dim = 1, 64
+    cfg.efla.per_token_beta = cfg.efla.use_query = cfg.efla.normalize_qk = True
+    m = EflaLM(cfg, "cuda").eval()
+    bits = torch.tensor([[1.0 if t >> i & 1 else -1.0 for i in range(7)] for t in range(128)],
+                        device="cuda")
+    step = torch.tensor([4.0 / 2 ** i for i in range(7)], device="cuda")
+    with torch.no_grad():
+        m.embed_tokens.fill_(1.0)
+        m.embed_tokens[:, 1:8] = bits.bfloat16()
+        w = m.blocks[0].efla.w_qkv
+        w.zero_()
+        w[64, 0] = 1.0        # k = e_0
+        w[128:192, 0] = 1.0   # v = 1
+        w[192, 1:8] = step.bfloat16()
+    st = m.new_states(128)
+    assert decode.decode_tokens(m, torch.arange(128, device="cuda")[:, None], st) is not None
+    alpha = -torch.expm1(-torch.sigmoid(bits @ step))
+    assert torch.equal(st[0][:, 0, 0], alpha[:, None].expand(128, 64))
+
+
 def test_native_decode_hands_back_other_forms():
     m = _model(64, True, True, True)
     tok = torch.zeros(1, 1, dtype=torch.int64, device="cuda")
