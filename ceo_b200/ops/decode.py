@@ -23,11 +23,12 @@ MAX_ROWS = 128  # rows of one decode call (sequences, or tokens of one prompt)
 
 def _hooked(*mods) -> bool:
     return any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks
-               or m._backward_pre_hooks or "forward" in m.__dict__ for m in mods)
+               or m._backward_pre_hooks or "forward" in m.__dict__ or "decode_step" in m.__dict__
+               for m in mods)
 
 
 def _dense(w, shape, dev) -> bool:
-    return (w.dtype is torch.bfloat16 and w.shape == shape and w.device == dev
+    return (w is not None and w.dtype is torch.bfloat16 and w.shape == shape and w.device == dev
             and w.is_contiguous() and not w.data_ptr() & 15 and not hasattr(w, "fsdp_gather"))
 
 
@@ -61,9 +62,11 @@ def _form(model):
     f = _Form()
     f.weights, f.eps, form = [], norm.eps, None
     for blk in model.blocks:
+        if type(blk) is not M.Block:  # a wrapper, or anything else that takes a block's place
+            return None
         mods = blk._modules
-        ln1, ln2, efla, mlp = mods["ln1"], mods["ln2"], mods["efla"], mods["mlp"]
-        if (type(blk) is not M.Block or type(efla) is not M.EflaLayer or type(mlp) is not M.MLP
+        ln1, ln2, efla, mlp = (mods.get(k) for k in ("ln1", "ln2", "efla", "mlp"))
+        if (type(efla) is not M.EflaLayer or type(mlp) is not M.MLP
                 or type(ln1) is not M.Norm or type(ln2) is not M.Norm
                 or mods.get("prism") is not None or mlp.fp8 is not None or efla.fp8 is not None
                 or mlp.act != "swiglu" or _hooked(blk, ln1, ln2, efla, mlp)
@@ -71,8 +74,11 @@ def _form(model):
                 or ln2.eps != f.eps):
             return None
         ep, mp = efla._parameters, mlp._parameters
-        n1, n2 = ln1._parameters["weight"], ln2._parameters["weight"]
-        w_qkv, w_o, w_up, w_down = ep["w_qkv"], ep["w_o"], mp["w_up"], mp["w_down"]
+        n1, n2 = ln1._parameters.get("weight"), ln2._parameters.get("weight")
+        w_qkv, w_o = ep.get("w_qkv"), ep.get("w_o")
+        w_up, w_down = mp.get("w_up"), mp.get("w_down")
+        if w_qkv is None:
+            return None
         this = (efla.P, efla.normalize, efla.per_token_beta, w_qkv.shape[0], efla.H, efla.d)
         if form is None:
             form = this
@@ -86,8 +92,8 @@ def _form(model):
             return None
         beta = 0
         if not efla.per_token_beta:
-            bp = ep["beta_param"]
-            if bp.dtype is not torch.float32 or bp.numel() != 1 or bp.device != dev:
+            bp = ep.get("beta_param")
+            if bp is None or bp.dtype is not torch.float32 or bp.numel() != 1 or bp.device != dev:
                 return None
             beta = bp.data_ptr()
         f.weights.append([n1.data_ptr(), w_qkv.data_ptr(), w_o.data_ptr(), n2.data_ptr(),

@@ -135,3 +135,50 @@ def test_native_decode_hands_back_other_forms():
     for i in ids:
         lb = m.decode_step(torch.tensor([i], device="cuda"), b)
     assert (la - lb).norm() / lb.norm() < 2e-2
+
+
+class _Wrapped(torch.nn.Module):
+    """A block behind another module, as a checkpointing or logging wrapper puts it."""
+
+    def __init__(self, blk):
+        super().__init__()
+        self.inner = blk
+
+    def forward(self, *a, **k):
+        return self.inner(*a, **k)
+
+    @property
+    def prism(self):
+        return self.inner.prism
+
+    @property
+    def dropout(self):
+        return self.inner.dropout
+
+    def decode_step(self, *a, **k):
+        return self.inner.decode_step(*a, **k)
+
+
+@pytest.mark.parametrize("how", ["wrapped block", "weight as attribute", "decode_step replaced"])
+def test_models_with_replaced_parts_run_layer_by_layer(how):
+    m, plain = _model(64, True, True, True), _model(64, True, True, True)
+    if how == "wrapped block":
+        m.blocks[1] = _Wrapped(m.blocks[1])
+    elif how == "weight as attribute":
+        w = m.blocks[1].efla.w_qkv.detach().clone()
+        del m.blocks[1].efla.w_qkv
+        m.blocks[1].efla.w_qkv = w
+    else:
+        calls = []
+        real = m.blocks[1].efla.decode_step
+        m.blocks[1].efla.decode_step = lambda *a: (calls.append(0), real(*a))[1]
+    tok = torch.randint(0, 1000, (2, 64), device="cuda",
+                        generator=torch.Generator(device="cuda").manual_seed(4))
+    with torch.no_grad():
+        a, b = m(tok), plain(tok)
+    assert (a - b).norm() < 2e-2 * b.norm()
+    sa, sb = m.new_states(2), plain.new_states(2)
+    a, b = m.decode_step(tok[:, 0], sa), plain.decode_step(tok[:, 0], sb)
+    assert (a - b).norm() < 2e-2 * b.norm()
+    if how == "decode_step replaced":
+        assert len(calls) == 1
