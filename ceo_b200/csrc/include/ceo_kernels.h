@@ -120,7 +120,8 @@ int ceo_efla_prep_bwd_logits(const void* dqn, const void* dkn, const void* qn, c
  * ln2.weight, w_up (2F x hidden, gate / up rows interleaved), w_down, state (fp32 (B,H,D,D)),
  * scalar beta (fp32) or NULL (beta logits are columns P*H*D.. of the projection)}.  All weights
  * bf16, dense, 16-byte aligned.  ws: bf16 workspace of the sum over {hidden, hidden, n_proj,
- * H*D, F} of round_up(B*T*width, 128) elements.  Launches 2 + 7 * n_layers (+ 1) kernels. */
+ * H*D, F} of round_up(B*T*width, 128) elements.  Launches 1 + 7 * n_layers kernels,
+ * and 2 more with logits. */
 int ceo_decode_tokens(const long long* ids, const void* table, long long vocab,
                       void* const* layers, int n_layers, const void* final_norm, const void* head,
                       float* logits, void* ws, int B, int T, int hidden, int H, int D, int P,

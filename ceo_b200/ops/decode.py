@@ -178,5 +178,5 @@ def forward_hidden(model, tokens: torch.Tensor, states=None, resets=None):
         model.final_norm.weight.data_ptr(), out.data_ptr(), ws.data_ptr(), size, _lib.ptr(resets),
         B, T, D, H, d, f.P, f.n_proj, F, f.normalize, float(f.eps),
         _lib.status_word(dev).data_ptr(), _lib.stream()), "ceo_forward_tokens")
-    _lib.launch_count += 2 + n * (10 if segs > 1 else 9) + (n if segs > 1 else 0)
+    _lib.launch_count += 2 + n * (12 if segs > 1 else 10)  # spans: a map pass and a fold more
     return out, finals

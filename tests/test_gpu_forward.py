@@ -39,6 +39,34 @@ def test_native_forward_matches_layers(d, per_token, use_query, B, T, monkeypatc
     assert all(torch.equal(x, y) for x, y in zip(sa, sb))
 
 
+def _kernels(f):
+    """(kernels of this library that ran in f(), what the launch counter added)."""
+    from torch.profiler import ProfilerActivity, profile
+    f()
+    torch.cuda.synchronize()
+    n = _lib.launch_count
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        f()
+        torch.cuda.synchronize()
+    n = _lib.launch_count - n
+    return sum(e.device_type == torch.autograd.DeviceType.CUDA and "ceo::" in e.name
+               for e in prof.events()), n
+
+
+@pytest.mark.parametrize("T", [64, 2048])  # the plain recurrence and spans
+def test_launches_are_counted(T):
+    m = _model(128, True, True)
+    tok = torch.zeros(1, T, dtype=torch.int64, device="cuda")
+    assert (_lib.lib().ceo_efla_fwd_segments(1, T, 4, 128) > 1) == (T == 2048)
+    with torch.no_grad():
+        ran, counted = _kernels(lambda: decode.forward_hidden(m, tok))
+        assert ran == counted > 0
+        st = m.new_states(1)
+        for logits in (True, False):
+            ran, counted = _kernels(lambda: decode.decode_tokens(m, tok[:, :5], st, logits))
+            assert ran == counted > 0
+
+
 def test_native_forward_hands_back_other_forms():
     m = _model(64, True, True)
     tok = torch.zeros(1, 64, dtype=torch.int64, device="cuda")
