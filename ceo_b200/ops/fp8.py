@@ -194,13 +194,7 @@ class Fp8LinearState:
 
     def weight_q(self, weight: torch.Tensor) -> torch.Tensor:
         if self.wq is None or self.wq_step != self.recipe.step_id:
-            if self.recipe.dgrad and weight.requires_grad \
-                    and weight.shape[0] % 16 == 0 and weight.shape[1] % 16 == 0:
-                # the backward pass will want the transposed codes: one read gives both
-                self.wq, self.wtq = quantize_t(weight.detach(), self.w_meta)
-                self.wtq_step = self.recipe.step_id
-            else:
-                self.wq = quantize(weight.detach(), self.w_meta)
+            self.wq = quantize(weight.detach(), self.w_meta)
             self.wq_step = self.recipe.step_id
         return self.wq
 
@@ -208,9 +202,7 @@ class Fp8LinearState:
         """e4m3 codes of ``weight^T`` (in, out), on the scale of ``weight_q``."""
         if self.wtq is None or self.wtq_step != self.recipe.step_id:
             self.weight_q(weight)  # makes sure the weight's scale is calibrated
-            if self.wtq is not None and self.wtq_step == self.recipe.step_id:
-                return self.wtq
-            self.wtq = _quantize_raw(transpose2d(weight.detach()), self.w_meta)
+            self.wtq = quantize_t(weight.detach(), self.w_meta, want_q=False)[1]
             self.wtq_step = self.recipe.step_id
         return self.wtq
 

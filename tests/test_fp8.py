@@ -149,3 +149,18 @@ def test_recipe_state_roundtrip():
     y1 = F8.fp8_linear(x, w, st)
     y2 = F8.fp8_linear(x, w, st2)
     assert torch.equal(y1, y2)
+
+
+def test_transposed_weight_codes_exist_only_once_a_gradient_asks():
+    # evaluation of a model whose data gradients are 8-bit: no backward pass, no second set of codes
+    torch.manual_seed(3)
+    w = (torch.randn(48, 32) * 0.1).requires_grad_()
+    st = F8.Fp8Recipe(dgrad=True).new_state("cpu")
+    x = torch.randn(16, 32, requires_grad=True)
+    with torch.no_grad():
+        F8.fp8_linear(x, w, st)
+    assert st.wq is not None and st.wtq is None
+    y = F8.fp8_linear(x, w, st)
+    assert st.wtq is None  # made, and its memory taken, where activations are being freed
+    y.sum().backward()
+    assert torch.equal(st.wtq, st.wq.t())
