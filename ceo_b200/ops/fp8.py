@@ -225,18 +225,23 @@ class Fp8Recipe:
     def step(self) -> None:
         metas = [m for st in self.states for m in (st.x_meta, st.w_meta, st.g_meta)
                  if m.calibrated]
-        if metas and metas[0].scale.is_cuda:
-            for i in range(0, len(metas), 64):  # 64 tensors a launch
-                part = metas[i:i + 64]
-                ptrs = (ctypes.c_void_p * (4 * len(part)))(*(
-                    t.data_ptr() for m in part for t in (m.history, m.cursor, m.amax, m.scale)))
-                fmax = (ctypes.c_float * len(part))(*(_FMAX[m.kind] for m in part))
-                _lib.check(_lib.lib().ceo_fp8_update_scales(
-                    ptrs, fmax, len(part), self.history, 2.0 ** self.margin, _lib.stream()),
-                    "ceo_fp8_update_scales")
-        else:
-            for m in metas:
-                m.update()
+        # 64 tensors a launch, as far as they share a device, this recipe's history and its margin
+        alike, rest = [], []
+        for m in metas:
+            dev = alike[0].scale.device if alike else m.scale.device
+            ok = (m.scale.is_cuda and m.scale.device == dev and m.margin == self.margin
+                  and m.history.numel() == self.history)
+            (alike if ok else rest).append(m)
+        for i in range(0, len(alike), 64):
+            part = alike[i:i + 64]
+            ptrs = (ctypes.c_void_p * (4 * len(part)))(*(
+                t.data_ptr() for m in part for t in (m.history, m.cursor, m.amax, m.scale)))
+            fmax = (ctypes.c_float * len(part))(*(_FMAX[m.kind] for m in part))
+            _lib.check(_lib.lib().ceo_fp8_update_scales(
+                ptrs, fmax, len(part), self.history, 2.0 ** self.margin, _lib.stream()),
+                "ceo_fp8_update_scales")
+        for m in rest:
+            m.update()
         self.step_id += 1
 
     def invalidate(self) -> None:

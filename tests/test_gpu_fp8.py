@@ -190,3 +190,32 @@ def test_fp8_convergence_tool_runs_both_arms(capsys):
     rec = json.loads(capsys.readouterr().out.strip().splitlines()[-1])
     assert rec["steps"] == 6 and abs(rec["loss_first"][0] - rec["loss_first"][1]) < 0.2
     assert abs(rec["rel_gap"]) < 0.05
+
+
+def test_recipe_step_over_unlike_metas():
+    # more tensors than one launch holds, some with a history, a margin or a device of their own
+    from ceo_b200.ops import fp8 as F8
+    torch.manual_seed(11)
+    rec, one_by_one = F8.Fp8Recipe(4, 1), []
+    for i in range(24):
+        st = rec.new_state(DEV)
+        for j, kind in enumerate(("x_meta", "w_meta", "g_meta")):
+            m = getattr(st, kind)
+            if (i + j) % 7 == 1:
+                m = F8.Fp8Meta("cpu" if i % 2 else DEV, m.kind, history=3 if j else 16, margin=1)
+            elif (i + j) % 7 == 2:
+                m = F8.Fp8Meta(DEV, m.kind, history=4, margin=3)
+            setattr(st, kind, m)
+            m.calibrated = (i + j) % 5 != 3
+            twin = F8.Fp8Meta(m.device, m.kind, m.history.numel(), m.margin)
+            one_by_one.append((m, twin))
+    for step in range(6):
+        for m, twin in one_by_one:
+            m.amax.fill_(float(torch.rand(()) * 3 + step))
+            twin.amax.copy_(m.amax)
+            if m.calibrated:
+                twin.update()
+        rec.step()
+    for m, twin in one_by_one:
+        assert torch.equal(m.scale, twin.scale) and torch.equal(m.history, twin.history)
+        assert torch.equal(m.cursor, twin.cursor) and torch.equal(m.amax, twin.amax)
