@@ -1244,9 +1244,29 @@ struct TilePick {
   int tn = 256, split = 1;
   bool pair = false;
 };
+// Whether an accumulation may be cut in K at all.  Slices meet in arrival order, so a cut product
+// does not repeat bit for bit; one is cut only where the 128 x 256 tiles, a wave at a time, leave
+// clearly more of the chip idle than two or three slices of at least 16 k-blocks would.  That is
+// narrower than what is faster (2048 x 2048 x 32768 fills 128 of 148 SMs and stays whole: 292 us
+// against 210 us in two slices): a caller's sums do not become order-dependent for 15 % of idle SMs.
+static bool may_cut(int M, int N, int num_kb, int batch, int cap) {
+  const long long tiles = static_cast<long long>((M + BM - 1) / BM) * ((N + BN - 1) / BN) * batch;
+  double best = 0.0;
+  bool cut = false;
+  for (int s = 1; s <= 3 && s * 16 <= num_kb; ++s) {
+    const long long units = tiles * s, waves = (units + cap - 1) / cap;
+    const double eff = static_cast<double>(units) / (waves * cap) - 0.05 * (s - 1);
+    if (eff > best + (s > 1 ? 0.05 : 0.0)) {
+      best = eff;
+      cut = s > 1;
+    }
+  }
+  return cut;
+}
 static TilePick pick_tiles(int M, int N, int num_kb, int batch, int cap, bool may_split) {
   TilePick best;
   double best_t = 1e30;
+  may_split = may_split && may_cut(M, N, num_kb, batch, cap);
   for (int kind = 0; kind < 3; ++kind) {  // 0: 128 x 256, 1: pair, 2: 128 x 128
     const int tm = kind == 1 ? 2 * BM : BM, tn = kind == 2 ? 128 : 256;
     const int slots = kind == 1 ? cap / 2 : cap;
@@ -1507,6 +1527,15 @@ extern "C" int ceo_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   return gemm_run(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, batch, batch_stride_a,
                   batch_stride_b, batch_stride_c, out_f32, accumulate, alpha, bias, residual, ldr,
                   batch_stride_r, status, max_ctas, fz, stream);
+}
+
+// How a plain product of this shape runs on a chip of `sms` SMs: 4 x K-slices + tile kind (0: 128 x
+// 256, 1: 256 x 256 on a CTA pair, 2: 128 x 128).  Up to 128 rows the few-row kernel comes first.
+extern "C" int ceo_gemm_pick(int M, int N, int K, int batch, int fp8, int accumulate, int sms) {
+  if (M < 1 || N < 1 || K < 1 || batch < 1 || sms < 1) return -5;
+  const int bke = fp8 ? 2 * ceo::BK : ceo::BK;
+  const ceo::TilePick t = ceo::pick_tiles(M, N, (K + bke - 1) / bke, batch, sms, accumulate != 0);
+  return 4 * t.split + (t.pair ? 1 : t.tn == 128 ? 2 : 0);
 }
 
 // C[b] = alpha * A[b] B[b]^T + beta * R[b], all bf16 (the Newton-Schulz update).

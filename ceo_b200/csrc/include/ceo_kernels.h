@@ -44,6 +44,10 @@ int ceo_gemm_bf16_axpy(const void* A, const void* B, void* C, int M, int N, int 
                        long long batch_stride_c, float alpha, float beta, const void* R,
                        long long ldr, long long batch_stride_r, int* status, cudaStream_t stream);
 
+/* Tile kind and K-slices that a plain product gets (host arithmetic only): 4 * slices + kind, kind
+ * 0: 128 x 256, 1: 256 x 256 on a CTA pair, 2: 128 x 128. */
+int ceo_gemm_pick(int M, int N, int K, int batch, int fp8, int accumulate, int sms);
+
 /* 1: weight-gradient GEMMs never split K (split-K accumulates with fp32 atomics, whose order
  * varies from run to run).  Default 0. */
 int ceo_set_deterministic(int on);

@@ -1,0 +1,50 @@
+"""The choice of tile shape and K-slices of a plain product (host arithmetic of the library)."""
+import random
+
+import pytest
+
+from ceo_b200.ops import _lib
+
+pytestmark = pytest.mark.skipif(not _lib.available(), reason="kernel library not built")
+
+
+def _pick(M, N, K, batch=1, fp8=0, accumulate=1, sms=148):
+    r = _lib.lib().ceo_gemm_pick(M, N, K, batch, fp8, accumulate, sms)
+    assert r >= 4
+    return r & 3, r >> 2
+
+
+def _fills_badly(M, N, kb, batch, sms):
+    """The 128 x 256 tiles leave so much of the last wave idle that two or three slices of at least
+    16 k-blocks would fill 5 % more, after 5 % for every extra slice."""
+    tiles, best, cut = -(-M // 128) * -(-N // 256) * batch, 0.0, False
+    for s in range(1, 4):
+        if s * 16 <= kb:
+            waves = -(-tiles * s // sms)
+            eff = tiles * s / (waves * sms) - 0.05 * (s - 1)
+            if eff > best + (0.05 if s > 1 else 0.0):
+                best, cut = eff, s > 1
+    return cut
+
+
+def test_only_products_that_fill_the_chip_badly_are_cut():
+    # slices meet in arrival order: every other accumulation repeats bit for bit
+    rng = random.Random(1)
+    log = lambda lo, hi: int(2 ** rng.uniform(lo, hi))
+    cut = 0
+    for _ in range(20000):
+        M, N, K, fp8 = log(3, 15), log(3, 15), log(6, 17), rng.randint(0, 1)
+        batch, sms = rng.choice((1, 1, 1, 3, 40)), rng.choice((148, 148, 100, 1))
+        kb = -(-K // (128 if fp8 else 64))
+        kind, slices = _pick(M, N, K, batch, fp8, 1, sms)
+        assert kind in (0, 1, 2) and (kind != 1 or sms >= 2)
+        if slices > 1:
+            assert _fills_badly(M, N, kb, batch, sms), (M, N, K, batch, fp8, sms)
+            per = -(-kb // slices)
+            assert slices <= 8 and per * (slices - 1) < kb  # no empty slice
+            cut += 1
+        assert _pick(M, N, K, batch, fp8, 0, sms)[1] == 1
+    assert cut > 1000
+    assert _pick(1024, 1024, 1984)[1] == 1      # 31 k-blocks
+    assert _pick(2048, 2048, 32768)[1] == 1     # 128 of 148 SMs
+    assert _pick(1024, 1024, 16384)[1] > 1      # 32 of 148 SMs
