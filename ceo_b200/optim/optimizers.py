@@ -301,9 +301,12 @@ class ShardedOptimizer:
                 for s in g:
                     self._muon_matrix(s, f.grads, lr, gscale)
                 continue
-            # at most 32 matrices (the kernels' pointer table) and 2^28 elements (512 MB of bf16
-            # per copy) at a time: by then every product fills the chip many times over
-            k = max(1, min(32, (1 << 28) // (shape[0] * shape[1])))
+            # at most 32 matrices (the kernels' pointer table) and 2^26 elements at a time, of
+            # which three bf16 copies (128 MB each) and the Gram matrices live at once.  Update of
+            # the 340M / 1.3B models' matrices and memory beside what the engine holds: one by one
+            # 29.7 / 67.2 ms, 0.20 / 0.40 GB; 2^25 elements 11.7 / 56.3 ms, 0.22 / 0.40 GB; 2^26
+            # 10.5 / 55.2 ms, 0.45 / 0.54 GB; 2^28 9.8 / 53.3 ms, 0.88 / 1.78 GB
+            k = max(1, min(32, (1 << 26) // (shape[0] * shape[1])))
             for i in range(0, len(g), k):
                 self._muon_group(g[i:i + k], lr, gscale)
 

@@ -74,3 +74,18 @@ def test_skipped_step_leaves_groups_alone():
     for n, st in opt._muon_state.items():
         for k, v in st.items():
             assert torch.equal(v, before[n][k])
+
+
+def test_groups_are_bounded_in_memory():
+    # 16 matrices of 2^24 elements: four at a time, three bf16 copies of them and four Gram matrices
+    m = _Mats([(4096, 4096)] * 16, 2)
+    flat = FlatParams(m)
+    opt = ShardedOptimizer(flat, "lion_muon", max_grad_norm=1.0)
+    flat.grads.normal_()
+    opt.step(0.1)  # momentum and masters exist from here on
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    opt.step(0.1)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - held < 4 * 2 * 2 ** 26 + 2 ** 24
