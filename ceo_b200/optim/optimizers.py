@@ -294,13 +294,14 @@ class ShardedOptimizer:
         f = self.flat
         groups = {}
         for s in segs:
-            groups.setdefault(s.shape, []).append(s)
+            # grouped kernels move 16 bytes at a time; a loaded state may be a slice of a buffer
+            if (self.cuda and f.param_dtype == torch.bfloat16 and f.grads.dtype == torch.float32
+                    and s.numel % 4 == 0
+                    and not any(t.data_ptr() & 15 for t in self._muon_state_of(s).values())):
+                groups.setdefault(s.shape, []).append(s)
+            else:
+                self._muon_matrix(s, f.grads, lr, gscale)
         for shape, g in groups.items():
-            if not (self.cuda and f.param_dtype == torch.bfloat16
-                    and f.grads.dtype == torch.float32 and shape[0] * shape[1] % 4 == 0):
-                for s in g:
-                    self._muon_matrix(s, f.grads, lr, gscale)
-                continue
             # at most 32 matrices (the kernels' pointer table) and 2^26 elements at a time, of
             # which three bf16 copies (128 MB each) and the Gram matrices live at once.  Update of
             # the 340M / 1.3B models' matrices and memory beside what the engine holds: one by one

@@ -89,3 +89,24 @@ def test_groups_are_bounded_in_memory():
     opt.step(0.1)
     torch.cuda.synchronize()
     assert torch.cuda.max_memory_allocated() - held < 4 * 2 * 2 ** 26 + 2 ** 24
+
+
+def test_state_loaded_from_slices_of_a_buffer():
+    # tensors of a state already on the device are taken as they are, whatever their alignment
+    shapes = [(64, 192)] * 3
+    out = []
+    for shift in (0, 1):
+        flat = FlatParams(_Mats(shapes, 5))
+        opt = ShardedOptimizer(flat, "lion_muon", max_grad_norm=1.0)
+        flat.grads.copy_(torch.sin(torch.arange(flat.total, device="cuda").float()))
+        opt.step(0.1)
+        st = opt.state_dict()
+        for one in st["muon"].values():
+            for k, t in one.items():
+                buf = torch.empty(t.numel() + 4, device="cuda")
+                one[k] = buf[shift:shift + t.numel()].copy_(t)
+        opt.load_state_dict(st)
+        flat.grads.copy_(torch.cos(torch.arange(flat.total, device="cuda").float()))
+        opt.step(0.1)
+        out.append(flat.params.float())
+    assert (out[0] - out[1]).abs().max() <= 2 ** -6
