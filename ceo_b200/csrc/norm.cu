@@ -564,8 +564,10 @@ extern "C" int ceo_rmsnorm_fwd(const void* x, const void* residual, const void* 
         xp, rp, wp, static_cast<bf16*>(y), static_cast<bf16*>(h_out), rstd, rows, eps);    \
     return static_cast<int>(cudaGetLastError());                                           \
   }
-  if (D == 512) CEO_RMS_FWD(64, 1)
-  if (D == 1024) CEO_RMS_FWD(128, 1)
+  // these two round x + residual to the stored h; without an h the general kernel keeps fp32 sums
+  const bool sums_stored = !residual || h_out;
+  if (D == 512 && sums_stored) CEO_RMS_FWD(64, 1)
+  if (D == 1024 && sums_stored) CEO_RMS_FWD(128, 1)
   if (D == 2048) CEO_RMS_FWD(256, 1)
   if (D == 4096) CEO_RMS_FWD(256, 2)
 #undef CEO_RMS_FWD

@@ -25,7 +25,7 @@ def test_few_rows_gemm(M, N, K):
     assert (got.double() - 0.5 * want).abs().max() <= 2 ** -18 * K ** 0.5 * 8
     got = matmul.gemm(a, w, residual=res)
     want = want + res.double()
-    # one rounding to bf16 (half an ulp, 2^-9 relative) plus the fp32 error
+    # one rounding to bf16 (half an ulp, 2^-8 relative) plus the fp32 error
     assert ((got.double() - want).abs() <= want.abs() * 2 ** -8 + 2 ** -15 * K ** 0.5).all()
 
 

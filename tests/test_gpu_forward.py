@@ -211,3 +211,19 @@ def test_rmsnorm_rows(D, rows):
         assert ((xs.grad.double() - hd.grad).abs() <= hd.grad.abs() * 2 ** -8 + 1e-4).all()
         assert ((ws.grad.double() - wd.grad).abs()
                 <= wd.grad.abs() * 2 ** -8 + 1e-5 * rows ** 0.5).all()
+
+
+@pytest.mark.parametrize("D", [512, 768, 1024])
+def test_rmsnorm_of_a_sum_that_is_not_stored(D):
+    # without an h to store, x + residual is normalised in fp32 at these widths
+    g = torch.Generator(device="cuda").manual_seed(D)
+    x, r, w = (torch.randn(n, D, device="cuda", generator=g).bfloat16() for n in (300, 300, 1))
+    y, rstd = torch.empty_like(x), torch.empty(300, device="cuda")
+    _lib.check(_lib.lib().ceo_rmsnorm_fwd(
+        x.data_ptr(), r.data_ptr(), w.data_ptr(), y.data_ptr(), None, rstd.data_ptr(), 300, D, 1e-6,
+        _lib.stream()), "ceo_rmsnorm_fwd")
+    h = x.double() + r.double()
+    want = h * torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    # one rounding to bf16 (half an ulp: 2^-8 of the power of two below) of an fp32 result
+    half_ulp = torch.ldexp(torch.ones_like(want), torch.frexp(want).exponent - 9)
+    assert ((y.double() - want).abs() <= half_ulp + want.abs() * 2 ** -20).all()

@@ -98,7 +98,7 @@ def _swiglu_case(M, F, D):
     matmul._gemm_swiglu(x, w, gu, M, 2 * F, D, False, 1, act)
     z = x.double() @ w.double().t()
     ref = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
-    # one bf16 rounding (2^-9 relative) of fp32 results; the exponential's own error stays below
+    # one bf16 rounding (2^-8 relative) of fp32 results; the exponential's own error stays below
     assert ((gu.double() - z).abs() <= z.abs() * 2 ** -8 + 1e-5).all()
     assert ((act.double() - ref).abs() <= ref.abs() * 2 ** -8 + 1e-4).all()
     dy = torch.randn(M, D, device="cuda", generator=g).bfloat16()
