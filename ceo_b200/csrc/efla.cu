@@ -1415,13 +1415,25 @@ static int efla_state_segmented(const CUtensorMap* m, const EflaTensors& t, int 
 }
 
 // Spans for a forward call: as many as keep the map pass (2 (D / 64) CTAs per span and chain)
-// within the two CTAs per SM that are resident, at least 6 chunks each; 1 (the plain kernel)
-// below three, where the extra passes eat the gain.
+// within the two CTAs per SM that are resident, at least 6 chunks each and at least three, if
+// that is 5 % less than the plain kernel by this estimate in microseconds.  Fitted to 1 to 74
+// chains of 6 to 1024 chunks with 3 to 40 spans (within 3 % at D = 64, 5 % at 128): a chunk's step
+// with one CTA per SM and with two, the plain kernel's step, a span's turn in the fold, and the
+// spans' matrices through memory.  Without it 16 to 32 chains of 128 and a few dozen chunks were
+// slower in spans than plain: 32 chains, 18 chunks, 71 us plain and 96 us in spans; 16 chains,
+// 18 chunks, 52 and 61 us; 16 chains, 64 chunks, 171 and 153 us (whole forward call).
 static int efla_segments(int B, int T, int H, int D) {
-  const int n = T / CH, per_span = 2 * (D / BV) * B * H;
-  int g = 1 + 296 / per_span;
+  const int n = T / CH, cols = D / BV;
+  const long long chains = static_cast<long long>(B) * H;
+  long long g = 1 + 296 / (2 * cols * chains);
   if (g > n / 6) g = n / 6;
-  return g >= 3 ? g : 1;
+  if (g < 3) return 1;
+  const double one = D == 64 ? 1.15 : 1.75, two = D == 64 ? 1.65 : 2.6, plain = D == 64 ? 1.23 : 1.8;
+  const double fold = D == 64 ? 1.0 : 3.0, cell = D == 64 ? 7.3e-6 : 12.7e-6;
+  const long long steps = (n + g - 1) / g, map = cols * chains * (2 * g - 3), real = cols * chains * g;
+  const double t = steps * ((map <= 148 ? one : two) + (real <= 148 ? one : two)) +
+                   fold * (g - 1) + cell * g * chains * D * D + 3.0;
+  return t < 0.95 * plain * n ? static_cast<int>(g) : 1;
 }
 
 template <int D>

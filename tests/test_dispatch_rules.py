@@ -1,4 +1,4 @@
-"""The choice of tile shape and K-slices of a plain product (host arithmetic of the library)."""
+"""Rules by which the library picks a kernel (host arithmetic, no GPU)."""
 import random
 
 import pytest
@@ -48,3 +48,20 @@ def test_only_products_that_fill_the_chip_badly_are_cut():
     assert _pick(1024, 1024, 1984)[1] == 1      # 31 k-blocks
     assert _pick(2048, 2048, 32768)[1] == 1     # 128 of 148 SMs
     assert _pick(1024, 1024, 16384)[1] > 1      # 32 of 148 SMs
+
+
+def test_spans_only_where_they_were_measured_faster():
+    spans = lambda chains, n, d: _lib.lib().ceo_efla_fwd_segments(1, 64 * n, chains, d)
+    # (chains, chunks, head size): plain faster by 2 % or more, spans faster by 2 % or more
+    plain = [(32, 18, 128), (32, 64, 128), (32, 128, 128), (24, 24, 128), (20, 32, 128),
+             (16, 18, 128), (16, 24, 128), (16, 32, 128), (12, 24, 128), (74, 32, 64), (64, 18, 64),
+             (32, 18, 64), (40, 24, 64), (1, 12, 64), (148, 1024, 64)]
+    spanned = [(16, 64, 128), (16, 128, 128), (8, 32, 128), (2, 64, 128), (24, 256, 128),
+               (16, 1024, 64), (16, 24, 64), (1, 18, 64), (32, 64, 64), (4, 18, 64)]
+    assert [s for s in plain if spans(*s) != 1] == []
+    assert [s for s in spanned if spans(*s) < 3] == []
+    for chains in (1, 7, 16, 33, 148, 1000):
+        for n in (1, 5, 17, 18, 100, 1023):
+            for d in (64, 128):
+                g = spans(chains, n, d)
+                assert g == 1 or (3 <= g <= n // 6 and (g - 1) * 2 * d // 64 * chains <= 296)
