@@ -6,8 +6,11 @@
 //   warp 0      TMA producer (one lane)
 //   warp 1      TMEM allocation + MMA issue (one lane)
 //   warps 2..5  epilogue (each owns one 32-lane TMEM quadrant)
-// Two 128x256 fp32 accumulators (all 512 TMEM columns) are double-buffered so
-// the epilogue of tile i overlaps the main loop of tile i+1.
+// Two fp32 accumulators are double-buffered in TMEM so that the epilogue of tile i
+// overlaps the main loop of tile i+1.  A plain product runs on one of three tiles
+// (pick_tiles): 128 x 256 of one CTA (both accumulators fill all 512 columns), 256 x
+// 256 of a CTA pair (cta_group::2) or 128 x 128; one of up to 128 rows goes to the
+// few-row kernel (skinny.cu).  The collectives use the 128 x 256 tile.
 //
 // Replaces the library GEMM + separate bias / column-sum kernels of the
 // reference (kernels/cuda/gemm.cu:182-234, 50-72) with one fused kernel.
@@ -1228,18 +1231,18 @@ static cudaError_t launch(int tn, bool pair, const CUtensorMap& ta, const CUtens
                    : launch_tn<A_MN, B_MN, FP8, 256>(ta, tb, p, grid, stream);
 }
 
-// Tile shape and K-slices of a plain product, in units of one k-block of a 128 x 256 tile
-// (0.40 us).  Measured per k-block: 1.0 for that tile, 0.9 for a 256 x 256 tile on a CTA pair,
-// 0.75 for a 128 x 128 tile (its MMA reads as many operand bytes per cycle as shared memory
-// gives; it wins where it fills SMs the wide ones leave idle).  Units run in waves of `cap` CTAs
-// or cap / 2 pairs.  32768 x 6208 x 2048: 570 us single, 535 us on pairs, 804 us 128-wide;
-// 576 x 2048 x 5632: 44 / 38 / 36 us.
-// An fp32 accumulation may be cut in K, its slices meeting through vector reductions.  That pays
-// where one wave leaves SMs idle or all CTAs walk K in lockstep (a lone full wave runs its
-// k-blocks about 1.3 times slower: 2048 x 2048 x 32768 292 us whole, 210 us in two slices;
-// 1024 x 1024 x 16384 110 us whole, 41 us in four); with many waves it loses (32000 x 2048 x
-// 16384: 1.49 ms whole, 1.64 ms in two, 2.4 ms in eight), since a unit cannot be shorter than
-// its epilogue (about 30 blocks).
+// Tile shape and K-slices of a plain product, by the predicted microseconds of its busiest CTA: the
+// main loop of the first tile, then for each further tile the longer of its main loop and the
+// epilogue that runs beside it, then the last epilogue.  Fitted to 1700 products in all three kinds
+// (M, N from 32 to 20000, K from 32 to 16384, batches to 24) and 200 accumulations in up to eight
+// slices.  A k-block (64 deep, 128 for 8-bit operands) of a 128 x 256 tile takes 0.48 us, of a 256 x
+// 256 tile on a CTA pair 0.385, of a 128 x 128 tile 0.363 (its MMA reads as many operand bytes per
+// cycle as shared memory gives).  What counts beside that is the epilogue: with a short K it is all
+// there is, and a pair's is 0.65 us longer since both CTAs have to free the accumulator.  The rule's
+// choice takes 0.4 % longer than the best kind in the mean and 0.85 of the 128 x 256 tile's time;
+// more than 2 % longer than the latter in 16 of the 1700.  32768 x 6208 x 2048: 570 us single, 535 us
+// on pairs, 804 us 128-wide; 7280 x 11928 x 40: 57 / 82 / 77 us; 576 x 2048 x 5632: 44 / 38 / 36 us;
+// 1024 x 1024 x 2176 accumulated: 21.3 us whole, 11.6 us in four slices of 128 x 256 tiles.
 struct TilePick {
   int tn = 256, split = 1;
   bool pair = false;
@@ -1263,25 +1266,29 @@ static bool may_cut(int M, int N, int num_kb, int batch, int cap) {
   }
   return cut;
 }
-static TilePick pick_tiles(int M, int N, int num_kb, int batch, int cap, bool may_split) {
+// Epilogues by what they move per 128 x 256 tile: bf16 stored; bf16 with a residual, SwiGLU forward
+// or fp32 stored; SwiGLU backward; fp32 accumulated (in slices: vector reductions); everything else
+// (rows that are no multiple of 16 bytes, bias ...), a row per lane.
+enum EpiCost { EPI_STORE = 0, EPI_MORE, EPI_SWIGLU_BWD, EPI_ACCUMULATE, EPI_GENERAL };
+static TilePick pick_tiles(int M, int N, int num_kb, int batch, int cap, int epi, bool may_split) {
+  static const double epi_us[5] = {3.4, 5.2, 9.6, 8.2, 36.0}, kb_us[3] = {0.48, 0.385, 0.363};
   TilePick best;
   double best_t = 1e30;
   may_split = may_split && may_cut(M, N, num_kb, batch, cap);
   for (int kind = 0; kind < 3; ++kind) {  // 0: 128 x 256, 1: pair, 2: 128 x 128
     const int tm = kind == 1 ? 2 * BM : BM, tn = kind == 2 ? 128 : 256;
     const int slots = kind == 1 ? cap / 2 : cap;
-    const double c = kind == 0 ? 1.0 : kind == 1 ? 0.9 : 0.75;
     if (slots < 1 || (kind == 1 && M <= BM)) continue;
     const long long tiles = static_cast<long long>((M + tm - 1) / tm) * ((N + tn - 1) / tn) * batch;
     for (int s = 1; s <= (may_split ? 8 : 1) && (s == 1 || s * 8 <= num_kb); ++s) {
       const int kb = (num_kb + s - 1) / s;
       if (s > 1 && static_cast<long long>(kb) * (s - 1) >= num_kb) continue;  // an empty slice
       const long long waves = (tiles * s + slots - 1) / slots;
-      double unit = c * kb;
-      if (may_split && waves == 1 && tiles * s * 2 > slots) unit *= 1.3;
-      if (s > 1 && waves > 1 && unit < 30.0) unit = 30.0;
-      const double t = s > 1 ? 1.07 * waves * unit + 30.0 : waves * unit + 8.0;
-      if (t < best_t * 0.98) {  // a near tie keeps the earlier kind and fewer slices
+      const double full = s > 1 && epi == EPI_ACCUMULATE ? 6.2 : epi_us[epi];
+      const double e = kind == 0 ? full : kind == 1 ? full + 0.65 : 0.63 * full;
+      const double loop = kb_us[kind] * kb;
+      const double t = 2.85 + loop + (waves - 1) * (loop > e ? loop : e) + e;
+      if (t < best_t * 0.97) {  // a near tie keeps the earlier kind and fewer slices
         best_t = t;
         best.tn = tn;
         best.split = s;
@@ -1355,7 +1362,14 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   TilePick pick;
   if (fz.kind == 0) {
     const int bke = f8.on ? 2 * BK : BK;
-    pick = pick_tiles(M, N, (K + bke - 1) / bke, batch, cap,
+    int cost = EPI_GENERAL;  // as the epilogue branches
+    if (epi.mode == 2) cost = EPI_SWIGLU_BWD;
+    else if (epi.mode == 1) cost = EPI_MORE;
+    else if (!bias && !out_f32 && !accumulate && !((N | ldc) & 7) && !(residual && (ldr & 7)))
+      cost = residual ? EPI_MORE : EPI_STORE;
+    else if (!bias && out_f32 && !residual && !((N | ldc) & 3))
+      cost = accumulate ? EPI_ACCUMULATE : EPI_MORE;
+    pick = pick_tiles(M, N, (K + bke - 1) / bke, batch, cap, cost,
                       out_f32 && accumulate && !bias && !residual && split_k_mode != 0 &&
                           !ceo::g_deterministic);
   }
@@ -1530,11 +1544,13 @@ extern "C" int ceo_gemm_bf16(const void* A, const void* B, void* C, int M, int N
 }
 
 // How a plain product of this shape runs on a chip of `sms` SMs: 4 x K-slices + tile kind (0: 128 x
-// 256, 1: 256 x 256 on a CTA pair, 2: 128 x 128).  Up to 128 rows the few-row kernel comes first.
-extern "C" int ceo_gemm_pick(int M, int N, int K, int batch, int fp8, int accumulate, int sms) {
-  if (M < 1 || N < 1 || K < 1 || batch < 1 || sms < 1) return -5;
+// 256, 1: 256 x 256 on a CTA pair, 2: 128 x 128).  epi: EpiCost; 3 (accumulation) may be cut in K.
+// Up to 128 rows the few-row kernel comes first.
+extern "C" int ceo_gemm_pick(int M, int N, int K, int batch, int fp8, int epi, int sms) {
+  if (M < 1 || N < 1 || K < 1 || batch < 1 || sms < 1 || epi < 0 || epi > ceo::EPI_GENERAL) return -5;
   const int bke = fp8 ? 2 * ceo::BK : ceo::BK;
-  const ceo::TilePick t = ceo::pick_tiles(M, N, (K + bke - 1) / bke, batch, sms, accumulate != 0);
+  const ceo::TilePick t = ceo::pick_tiles(M, N, (K + bke - 1) / bke, batch, sms, epi,
+                                          epi == ceo::EPI_ACCUMULATE);
   return 4 * t.split + (t.pair ? 1 : t.tn == 128 ? 2 : 0);
 }
 

@@ -45,8 +45,9 @@ int ceo_gemm_bf16_axpy(const void* A, const void* B, void* C, int M, int N, int 
                        long long ldr, long long batch_stride_r, int* status, cudaStream_t stream);
 
 /* Tile kind and K-slices that a plain product gets (host arithmetic only): 4 * slices + kind, kind
- * 0: 128 x 256, 1: 256 x 256 on a CTA pair, 2: 128 x 128. */
-int ceo_gemm_pick(int M, int N, int K, int batch, int fp8, int accumulate, int sms);
+ * 0: 128 x 256, 1: 256 x 256 on a CTA pair, 2: 128 x 128.  epi: 0 bf16 store, 1 with residual, SwiGLU
+ * forward or fp32 store, 2 SwiGLU backward, 3 fp32 accumulation, 4 everything else. */
+int ceo_gemm_pick(int M, int N, int K, int batch, int fp8, int epi, int sms);
 
 /* 1: weight-gradient GEMMs never split K (split-K accumulates with fp32 atomics, whose order
  * varies from run to run).  Default 0. */

@@ -8,8 +8,11 @@ from ceo_b200.ops import _lib
 pytestmark = pytest.mark.skipif(not _lib.available(), reason="kernel library not built")
 
 
-def _pick(M, N, K, batch=1, fp8=0, accumulate=1, sms=148):
-    r = _lib.lib().ceo_gemm_pick(M, N, K, batch, fp8, accumulate, sms)
+STORE, MORE, SWIGLU_BWD, ACCUMULATE, GENERAL = range(5)  # epilogues
+
+
+def _pick(M, N, K, batch=1, fp8=0, epi=ACCUMULATE, sms=148):
+    r = _lib.lib().ceo_gemm_pick(M, N, K, batch, fp8, epi, sms)
     assert r >= 4
     return r & 3, r >> 2
 
@@ -36,18 +39,33 @@ def test_only_products_that_fill_the_chip_badly_are_cut():
         M, N, K, fp8 = log(3, 15), log(3, 15), log(6, 17), rng.randint(0, 1)
         batch, sms = rng.choice((1, 1, 1, 3, 40)), rng.choice((148, 148, 100, 1))
         kb = -(-K // (128 if fp8 else 64))
-        kind, slices = _pick(M, N, K, batch, fp8, 1, sms)
+        kind, slices = _pick(M, N, K, batch, fp8, ACCUMULATE, sms)
         assert kind in (0, 1, 2) and (kind != 1 or sms >= 2)
         if slices > 1:
             assert _fills_badly(M, N, kb, batch, sms), (M, N, K, batch, fp8, sms)
             per = -(-kb // slices)
             assert slices <= 8 and per * (slices - 1) < kb  # no empty slice
             cut += 1
-        assert _pick(M, N, K, batch, fp8, 0, sms)[1] == 1
+        assert _pick(M, N, K, batch, fp8, rng.choice((STORE, MORE, SWIGLU_BWD, GENERAL)), sms)[1] == 1
     assert cut > 1000
     assert _pick(1024, 1024, 1984)[1] == 1      # 31 k-blocks
     assert _pick(2048, 2048, 32768)[1] == 1     # 128 of 148 SMs
     assert _pick(1024, 1024, 16384)[1] > 1      # 32 of 148 SMs
+
+
+def test_tiles_no_slower_than_the_wide_ones():
+    # products with the microseconds of the 128 x 256 tile, of the pair and of the 128 x 128 tile: a
+    # short K and many tiles (epilogues are all there is), a long K, a lone wave, whole products
+    measured = [
+        (7280, 11928, 40, 1, STORE, (57.1, 82.0, 76.7)), (1800, 4096, 136, 16, STORE, (76.6, 102.4, 106.6)),
+        (4096, 1184, 104, 16, STORE, (56.1, 68.7, 74.9)), (15784, 6280, 304, 1, STORE, (81.8, 99.7, 98.0)),
+        (13712, 14480, 168, 1, STORE, (124.4, 167.8, 169.9)), (368, 4096, 96, 5, STORE, (10.5, 15.4, 12.4)),
+        (2472, 8616, 40, 1, MORE, (32.8, 37.1, 38.2)), (3184, 10520, 488, 1, STORE, (53.9, 46.1, 63.2)),
+        (5760, 1552, 232, 1, MORE, (19.2, 20.8, 16.6)), (3176, 1472, 272, 1, SWIGLU_BWD, (23.1, 25.0, 20.5)),
+        (32768, 6208, 2048, 1, STORE, (570.0, 535.0, 804.0)), (576, 2048, 5632, 1, STORE, (44.0, 38.0, 36.0))]
+    for M, N, K, batch, epi, us in measured:
+        kind, _ = _pick(M, N, K, batch, 0, epi)
+        assert us[kind] <= 1.02 * us[0], (M, N, K, batch, epi, kind)
 
 
 def test_spans_only_where_they_were_measured_faster():

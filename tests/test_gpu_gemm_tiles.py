@@ -7,28 +7,30 @@ from ceo_b200.ops import _lib, fp8, matmul
 
 pytestmark = pytest.mark.gpu
 WIDE, PAIR, NARROW = 0, 1, 2
+STORE, MORE, SWIGLU_BWD, ACCUMULATE, GENERAL = range(5)  # epilogues
 
 
-def _kind(M, N, K, batch=1, fp8=0, accumulate=0):
+def _kind(M, N, K, epi, batch=1, fp8=0):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    r = _lib.lib().ceo_gemm_pick(M, N, K, batch, fp8, accumulate, sms)
+    r = _lib.lib().ceo_gemm_pick(M, N, K, batch, fp8, epi, sms)
     return r & 3, r >> 2
 
 
-# last tiles that are ragged in M, N and K, a last CTA of a pair with no row at all (M = 264, 2312),
-# whole 64-column panels (320, 1216, 192), rows that are no multiple of 16 bytes (N = 11270 ...)
+# last tiles that are ragged in M, N and K, a last CTA of a pair with no row at all (M = 264, 520,
+# 2312), whole 64-column panels (320, 1216, 192), rows that are no multiple of 16 bytes (N = 11270 ...)
 SHAPES = [(WIDE, 264, 264, 520, 20), (WIDE, 264, 11272, 520, 1), (WIDE, 2312, 1032, 520, 3),
-          (WIDE, 320, 11264, 512, 1), (WIDE, 264, 11270, 520, 1), (PAIR, 200, 11272, 520, 1),
-          (PAIR, 1160, 2056, 520, 1), (PAIR, 2312, 1032, 520, 1), (PAIR, 264, 2056, 520, 3),
-          (PAIR, 200, 520, 520, 20), (PAIR, 1216, 2112, 520, 1), (PAIR, 1160, 2050, 520, 1),
-          (NARROW, 264, 520, 520, 1), (NARROW, 1000, 264, 520, 1), (NARROW, 200, 264, 520, 3),
-          (NARROW, 192, 320, 520, 1), (NARROW, 264, 518, 520, 1)]
+          (WIDE, 320, 11264, 512, 1), (WIDE, 264, 11270, 520, 1), (PAIR, 200, 11264, 1032, 1),
+          (PAIR, 1160, 2056, 1032, 1), (PAIR, 2312, 1032, 1032, 1), (PAIR, 264, 2056, 1032, 3),
+          (PAIR, 520, 4104, 1032, 1), (PAIR, 200, 520, 1032, 20), (PAIR, 1216, 2112, 1032, 1),
+          (PAIR, 520, 4102, 4104, 1), (NARROW, 264, 520, 520, 1), (NARROW, 1000, 264, 520, 1),
+          (NARROW, 200, 264, 520, 3), (NARROW, 192, 320, 520, 1), (NARROW, 264, 518, 520, 1)]
 
 
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("kind,M,N,K,batch", SHAPES)
 def test_every_tile_kind(kind, M, N, K, batch, a_mn, b_mn):
-    assert _kind(M, N, K, batch) == (kind, 1)
+    for epi in (GENERAL,) if N % 8 else (STORE, MORE, ACCUMULATE):
+        assert _kind(M, N, K, epi, batch) == (kind, 1)
     if b_mn and N % 8:
         pytest.skip("a TMA row stride is a multiple of 16 bytes")
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
@@ -45,16 +47,15 @@ def test_every_tile_kind(kind, M, N, K, batch, a_mn, b_mn):
     # fp32 sums of K unit-normal products in any order
     acc = new(M, N)
     w = want + acc.double()
-    assert _kind(M, N, K, batch, 0, 1) == (kind, 1)
     matmul.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=acc, accumulate=True)
     assert (acc.double() - w).abs().max() <= 2 ** -16 * K ** 0.5 * 4
 
 
-@pytest.mark.parametrize("kind,M,N,K", [(WIDE, 264, 1032, 4104), (WIDE, 520, 2056, 4104),
-                                        (PAIR, 520, 520, 4104), (PAIR, 2056, 264, 4104),
-                                        (NARROW, 2056, 36, 4104)])
+@pytest.mark.parametrize("kind,M,N,K", [(WIDE, 520, 2056, 4104), (WIDE, 1032, 1032, 8200),
+                                        (PAIR, 2056, 264, 4104), (PAIR, 520, 520, 16392),
+                                        (NARROW, 264, 1032, 4104), (NARROW, 2056, 36, 4104)])
 def test_k_slices_of_every_tile_kind(kind, M, N, K):
-    got, slices = _kind(M, N, K, accumulate=1)
+    got, slices = _kind(M, N, K, ACCUMULATE)
     assert got == kind and slices > 1
     g = torch.Generator(device="cuda").manual_seed(M + N)
     a, b = (torch.randn(K, n, device="cuda", generator=g).bfloat16() for n in (M, N + N % 8))
@@ -65,11 +66,11 @@ def test_k_slices_of_every_tile_kind(kind, M, N, K):
     assert (acc.double() - w).abs().max() <= 2 ** -16 * K ** 0.5 * 4
 
 
-@pytest.mark.parametrize("kind,M,N", [(WIDE, 264, 11272), (WIDE, 320, 11264), (PAIR, 1160, 2064),
-                                      (PAIR, 2312, 1040), (NARROW, 200, 528)])
-def test_every_tile_kind_on_8_bit_operands(kind, M, N):
-    K = 528
-    assert _kind(M, N, K, fp8=1)[0] == kind
+@pytest.mark.parametrize("kind,M,N,K", [
+    (WIDE, 264, 11272, 528), (WIDE, 320, 11264, 528), (PAIR, 1160, 2064, 2064),
+    (PAIR, 2312, 1040, 2064), (PAIR, 4360, 2064, 4112), (NARROW, 200, 528, 528)])
+def test_every_tile_kind_on_8_bit_operands(kind, M, N, K):
+    assert _kind(M, N, K, STORE, fp8=1)[0] == _kind(M, N, K, ACCUMULATE, fp8=1)[0] == kind
     g = torch.Generator(device="cuda").manual_seed(M + N)
     a, b = (torch.randn(n, K, device="cuda", generator=g).to(torch.float8_e4m3fn) for n in (M, N))
     want = a.float().double() @ b.float().double().t()
@@ -82,10 +83,11 @@ def test_every_tile_kind_on_8_bit_operands(kind, M, N):
 
 # both SwiGLU epilogues: (kind of the gate / up product, kind of the data gradient)
 @pytest.mark.parametrize("up,down,M,F,D", [
-    (PAIR, PAIR, 2312, 1376, 136), (PAIR, PAIR, 4360, 2816, 264), (PAIR, NARROW, 1160, 1376, 136),
-    (WIDE, PAIR, 8456, 1376, 72), (WIDE, WIDE, 264, 11296, 136), (NARROW, NARROW, 576, 1376, 136)])
+    (PAIR, PAIR, 2312, 1376, 1032), (PAIR, PAIR, 1160, 2816, 1032), (PAIR, WIDE, 4360, 2816, 1032),
+    (PAIR, NARROW, 1160, 1376, 1032), (WIDE, WIDE, 8456, 1376, 72), (WIDE, WIDE, 264, 11296, 136),
+    (NARROW, NARROW, 576, 1376, 136)])
 def test_swiglu_epilogues_of_every_tile_kind(up, down, M, F, D):
-    assert _kind(M, 2 * F, D) == (up, 1) and _kind(M, F, D) == (down, 1)
+    assert _kind(M, 2 * F, D, MORE) == (up, 1) and _kind(M, F, D, SWIGLU_BWD) == (down, 1)
     _swiglu_case(M, F, D)
 
 
