@@ -63,7 +63,9 @@ def test_k_slices_of_every_tile_kind(kind, M, N, K):
     acc = torch.randn(M, N, device="cuda", generator=g)
     w = a.double().t() @ b.double() + acc.double()
     matmul.gemm(a, b, a_mn=True, b_mn=True, out=acc, accumulate=True)
-    assert (acc.double() - w).abs().max() <= 2 ** -16 * K ** 0.5 * 4
+    # the tensor core drops what lies below its accumulator, at most 2^-22 of a sum of at most 6
+    # standard deviations, at each of its K / 16 steps; a slice's sums are shorter by its share
+    assert (acc.double() - w).abs().max() <= K / 16 * 2 ** -22 * 6 * (K / slices) ** 0.5
 
 
 @pytest.mark.parametrize("kind,M,N,K", [
