@@ -1436,8 +1436,11 @@ static int gemm_run(const void* A, const void* B, void* C, int M, int N, int K, 
   // 128-row tiles and K-slices that fill the chip: the 97 products of a 1.3B decode step (one
   // row, 2.4 GB of weights) take 0.97 ms one after the other, and 0.96 ms the whole step when
   // chained (decode.cu); it was 12 ms.
+  // Above 64 rows it loses where B's tiles outnumber the SMs (100 rows of 32000 x 2048: 31 us, here 28)
+  // and with a short K, where the exchange of partial sums is all there is (128 x 760 x 120: 11.2, 6.2).
+  const bool few_rows_lose = M > 64 && (N > 148 * 128 || K <= 512);
   if (fz.kind == 0 && !f8.on && !a_mn_major && !b_mn_major && batch == 1 && !accumulate && !bias &&
-      max_ctas <= 0 && M <= 128 && epi.mode != 2 && epi.res_scale == 1.f) {
+      max_ctas <= 0 && M <= 128 && !few_rows_lose && epi.mode != 2 && epi.res_scale == 1.f) {
     SkinnyArgs g = {};
     g.A = A; g.W = B; g.C = C; g.residual = residual; g.act = epi.mode == 1 ? epi.aux : nullptr;
     g.lda = lda; g.ldw = ldb; g.ldc = ldc; g.ldr = ldr; g.ldact = epi.ld_aux;
